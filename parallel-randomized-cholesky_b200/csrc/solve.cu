@@ -197,14 +197,27 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
     return false;
 }
 
+// Column sums of the blocks' partials by the whole last block: thread t adds
+// every (kBlock / K)-th partial of column t % K, then a fixed tree joins the
+// threads of a column (deterministic).  One thread per column adding all the
+// partials (1184 for the SpMV's grid) was a chain of L2 round trips: it took
+// 16 of the 23 us of a 2867-unknown SpMV launch.
 template <int K>
 __device__ void sum_partials(const double* part, int nblocks, double* out) {
-    // threads < K each sum one column in block order
-    if (threadIdx.x < K) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * K + threadIdx.x];
-        out[threadIdx.x] = s;
+    __shared__ double red[kBlock];
+    constexpr int G = kBlock / K;
+    const int c = threadIdx.x % K, g = threadIdx.x / K;
+    double s = 0.0;
+#pragma unroll 4
+    for (int b = g; b < nblocks; b += G) s += __ldcg(part + (size_t)b * K + c);
+    red[threadIdx.x] = s;
+    __syncthreads();
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+        if (g < o) red[threadIdx.x] += red[threadIdx.x + o * K];
+        __syncthreads();
     }
+    if (threadIdx.x < K) out[threadIdx.x] = red[threadIdx.x];
     __syncthreads();
 }
 
@@ -477,11 +490,11 @@ __global__ void __launch_bounds__(kBlock, 8) spmv_update_kernel(SolveArgs a) {
     block_partials_lane<K>(acc, a.part + (size_t)blockIdx.x * K);
     if (last_block(&a.sc->ticket[1])) {
         sum_partials<K>(a.part, gridDim.x, a.sc->pq);
-        if (threadIdx.x < K && a.n_lrows > 0) {
-            // the long rows' terms of column c, in row order
-            double t = 0.0;
-            for (int k = 0; k < a.n_lrows; ++k) t += a.lr_dot[(size_t)k * K + threadIdx.x];
-            a.sc->pq[threadIdx.x] += t;
+        if (a.n_lrows > 0) {
+            // the long rows' terms, summed the same way
+            double* t = a.lr_dot + (size_t)a.n_lrows * K;
+            sum_partials<K>(a.lr_dot, a.n_lrows, t);
+            if (threadIdx.x < K) a.sc->pq[threadIdx.x] += t[threadIdx.x];
         }
         if (threadIdx.x < K) {
             int c = threadIdx.x;
@@ -507,14 +520,11 @@ constexpr int kSpmvChunk = RCHOL_SPMV_CHUNK;  // entries staged per warp and chu
 // entry order, then the threads' sums in a fixed tree; the same q, p, y and
 // p.q term as the tile and sliced-ELL kernels, which skip these rows.
 
-// pq += the long rows' p.q terms (spmv_long_kernel ran first): each thread
-// every kBlock-th term in order, then the threads in a fixed tree.  Called
-// by every thread of the SpMV's last block.
+// pq += the long rows' p.q terms (spmv_long_kernel ran first), in a fixed
+// tree.  Called by every thread of the SpMV's last block.
 __device__ void add_long_row_terms(SolveArgs& a) {
     if (a.n_lrows == 0) return;
-    double lt[1] = {0.0};
-    for (int k = threadIdx.x; k < a.n_lrows; k += blockDim.x) lt[0] += a.lr_dot[k];
-    block_partials<1>(lt, a.lr_dot + a.n_lrows);
+    sum_partials<1>(a.lr_dot, a.n_lrows, a.lr_dot + a.n_lrows);
     if (threadIdx.x == 0) a.sc->pq[0] += a.lr_dot[a.n_lrows];
 }
 
@@ -1133,16 +1143,16 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) bwd_pack_kernel(Solve
     block_partials<1>(acc, a.part + (size_t)(2 * a.grid_max + blockIdx.x));
     if (last_block(&a.sc->ticket[3])) {
         sum_partials<1>(a.part + (size_t)2 * a.grid_max, gridDim.x, a.sc->pq);
+        double extra[1] = {0.0};
+        // split rows: every kBlock-th by one thread, then a fixed tree
+        for (int q = threadIdx.x; q < a.nsplit_b; q += kBlock) {
+            const int32_t j = a.srow_b[q];
+            extra[0] += a.r[j] * ld_relaxed_f64(a.z + j);
+        }
+        if (a.nsplit_b) block_partials<1>(extra, a.part);  // the SpMV's partials are done with
         if (threadIdx.x == 0) {
             if (a.hb_ntask > 0) a.sc->pq[0] += a.sc->hrz;
-            if (a.nsplit_b) {  // split rows in id order
-                double extra = a.sc->pq[0];
-                for (int q = 0; q < a.nsplit_b; ++q) {
-                    const int32_t j = a.srow_b[q];
-                    extra += a.r[j] * ld_relaxed_f64(a.z + j);
-                }
-                a.sc->pq[0] = extra;
-            }
+            if (a.nsplit_b) a.sc->pq[0] += a.part[0];
             bwd_scalars(a, 1);
         }
     }
@@ -1544,7 +1554,7 @@ class PcgSolver {
                 lr_dot = nullptr;
                 cap_lrows = 0;
                 e = cudaMalloc(&lrows, sizeof(int32_t) * (size_t)cnt);
-                if (e == cudaSuccess) e = cudaMalloc(&lr_dot, sizeof(double) * ((size_t)cnt * K + 1));
+                if (e == cudaSuccess) e = cudaMalloc(&lr_dot, sizeof(double) * ((size_t)cnt + 1) * K);
                 if (e == cudaSuccess) cap_lrows = cnt;
             }
             if (e == cudaSuccess) {
@@ -2013,26 +2023,26 @@ __device__ void chunk_store(double va, double vb, double* out /* [2][K] */) {
     __syncthreads();
 }
 
-// Sum of the chunk partials of every (system, column) pair into out[pair]:
-// one warp per pair, lanes over the system's chunks, fixed tree.
+// Sum of the chunk partials of every (system, column) pair into out[pair]: a
+// warp per system, column lane % K, 32 / K chunks per load, fixed tree.
 template <int K>
 __device__ void reduce_pairs(const BatchArgs& a, const double* part, double* out) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int pairs = a.nsys * K;
-    for (int pr = w; pr < pairs; pr += kBlock / 32) {
-        const int sys = pr / K, c = pr % K;
+    constexpr int S = 32 / K;
+    const int c = lane % K, g = lane / K;
+    for (int sys = w; sys < a.nsys; sys += kBlock / 32) {
         const int64_t r0 = a.sys_off[sys], r1 = a.sys_off[sys + 1];
         double t = 0.0;
         if (r1 > r0) {
             const int64_t c0 = r0 / a.chunk, c1 = (r1 - 1) / a.chunk;
-            for (int64_t ch = c0 + lane; ch <= c1; ch += 32) {
-                const int slot = a.seg[ch * a.chunk] == sys ? 0 : 1;
-                t += part[(size_t)ch * 2 * K + slot * K + c];
-            }
+            // a chunk that starts before the system holds it in its second slot
+#pragma unroll 8
+            for (int64_t ch = c0 + g; ch <= c1; ch += S)
+                t += __ldcg(part + (size_t)ch * 2 * K + (ch * a.chunk < r0 ? K : 0) + c);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-        if (lane == 0) out[pr] = t;
+        for (int o = 16; o >= K; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+        if (lane < K) out[sys * K + lane] = t;
     }
     __syncthreads();
 }
@@ -2069,17 +2079,17 @@ __global__ void __launch_bounds__(kBlock) batch_init_kernel(BatchArgs a) {
     }
     if (last_block(&a.sc->ticket[0])) {
         reduce_pairs<K>(a, a.part, a.s.bnorm2);
+        int any = 0;
         for (int pr = threadIdx.x; pr < a.nsys * K; pr += kBlock) {
             a.s.alpha[pr] = 0.0;
             a.s.beta[pr] = 0.0;
             a.s.rz[pr] = 0.0;
             a.s.active[pr] = a.s.bnorm2[pr] > 0.0 ? 1 : 0;
+            any |= a.s.bnorm2[pr] > 0.0;
             a.s.iters[pr] = 0;
         }
-        __syncthreads();
+        any = __syncthreads_or(any);
         if (threadIdx.x == 0) {
-            int any = 0;
-            for (int pr = 0; pr < a.nsys * K; ++pr) any |= a.s.active[pr];
             a.sc->done = any ? 0 : 1;
             a.sc->iter = 0;
             a.sc->phase = 0;
@@ -2149,6 +2159,7 @@ __global__ void __launch_bounds__(kBlock) batch_dots_kernel(BatchArgs a) {
         reduce_pairs<K>(a, part_rz, a.s.rzn);
         const bool init = a.sc->phase == 0;
         const int it = init ? a.sc->iter : a.sc->iter + 1;
+        int any = 0;
         for (int pr = threadIdx.x; pr < a.nsys * K; pr += kBlock) {
             if (!a.s.active[pr]) {
                 a.s.beta[pr] = 0.0;
@@ -2159,6 +2170,7 @@ __global__ void __launch_bounds__(kBlock) batch_dots_kernel(BatchArgs a) {
                 a.s.rz[pr] = rn;
                 a.s.rz0[pr] = rn;
                 a.s.beta[pr] = 0.0;
+                any = 1;
                 continue;
             }
             a.s.iters[pr] = it;
@@ -2170,11 +2182,10 @@ __global__ void __launch_bounds__(kBlock) batch_dots_kernel(BatchArgs a) {
             a.s.beta[pr] = ro != 0.0 ? rn / ro : 0.0;
             a.s.rz[pr] = rn;
             if (conv) a.s.active[pr] = 0;
+            else any = 1;
         }
-        __syncthreads();
+        any = __syncthreads_or(any);
         if (threadIdx.x == 0) {
-            int any = 0;
-            for (int pr = 0; pr < a.nsys * K; ++pr) any |= a.s.active[pr];
             a.sc->iter = it;
             a.sc->phase = 1;
             if (!any || it >= a.max_iter) a.sc->done = 1;
@@ -2286,8 +2297,15 @@ BatchSolver* batch_create(const DevCsc& A, const DevFactor& F, const SolveConfig
         case 32: bind_batch<32>(s); break;
         default: *err = cudaErrorInvalidValue; batch_destroy(s); return nullptr;
     }
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // enough chunks for 4 CTAs per SM, of at least 128 rows where the systems
+    // allow it (a 293 k-row batch of 12 systems: 72 chunks of 4096 rows left
+    // half of the SMs idle)
     int64_t chunk = 32;
-    while (chunk * 2 <= std::min<int64_t>(minsys, 4096)) chunk *= 2;
+    while (chunk * 2 <= std::min<int64_t>(minsys, 4096) &&
+           (chunk < 128 || A.n / (chunk * 2) >= (int64_t)sms * 4))
+        chunk *= 2;
     const int K = cfg.k;
     const int64_t pairs = (int64_t)nsys * K;
     BatchArgs& a = s->ba;
@@ -2338,8 +2356,6 @@ BatchSolver* batch_create(const DevCsc& A, const DevFactor& F, const SolveConfig
     a.s.rzn = P + 8 * pairs;
     a.s.active = s->ipool;
     a.s.iters = s->ipool + pairs;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     s->grid = (int)std::min<int64_t>(a.nchunks, (int64_t)sms * 8);
     return s;
 }
