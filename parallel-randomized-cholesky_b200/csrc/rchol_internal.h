@@ -84,9 +84,13 @@ struct DevCsc {
 };
 
 // Rows longer than kLongRow entries (the hubs of power-law graphs) are left
-// out of the one-RHS SpMV kernels' tiles and slices: each gets a CTA of its
-// own (spmv_long_kernel).
-constexpr int kLongRow = 2048;
+// out of the SpMV kernels' tiles and slices: each gets a CTA of its own
+// (spmv_long_kernel).  A warp walks its widest row 8 entries per round trip,
+// so the longest row kept in a slice bounds the launch: on a 100 k-vertex
+// Chung-Lu graph the one-RHS SpMV took 0.458 ms with 2048 and 0.121 ms with
+// 512 (rows of finite-element stencils, up to a few hundred entries, stay in
+// the slices).
+constexpr int kLongRow = 512;
 
 // Columns of the input longer than kHugeCol entries are counted by the whole
 // grid rather than one warp (count_lower, factor.cu); the list that carries
