@@ -122,6 +122,14 @@ void free_factor(DevFactor& f) {
     f = DevFactor();
 }
 
+// A factor that could not be completed: its buffers, and its place in the
+// context's list of live factors (rchol_destroy walks that list).
+void drop_factor(rchol_ctx* ctx, rchol_factor_t* f) {
+    ctx->live.erase(std::remove(ctx->live.begin(), ctx->live.end(), f), ctx->live.end());
+    free_factor(f->F);
+    delete f;
+}
+
 int64_t pow2_ge(int64_t x) {
     int64_t p = 1;
     while (p < x) p <<= 1;
@@ -133,6 +141,18 @@ bool has_device() {
     return cudaGetDeviceCount(&n) == cudaSuccess && n > 0;
 }
 
+// The last vertices eliminated by a CTA each rather than a warp: late vertices
+// gather the longest lists and sit in narrow levels, where a vertex's own
+// latency counts; early ones are many, and 592 CTAs take them slower than 3552
+// warps.  At least 16 k vertices, more for large matrices with longer columns,
+// at most an eighth.  Factor time (ms) with none / lnnz / 192 / 96 / 48 / 24 of
+// them: 128^3 7-point 12.9 / 9.9 / 9.4 / 9.5 / 10.3; 61x53x47 2.88 / 2.36 / 2.11
+// / 1.88 / 1.73; 27-point 72x70x67 106 / 23.1 / 20.7 / 20.7 / 20.7 (an eighth
+// from 96 on); 256^2 5-point 0.465 / 0.473 / 0.479 / 0.470 / 0.470.
+int32_t cta_vertices(int32_t n, int64_t lnnz) {
+    return (int32_t)std::min<int64_t>(n / 8, std::max<int64_t>(lnnz / 96, 16384));
+}
+
 // Sizes of the factor work pools.
 struct PoolPlan {
     int c0;
@@ -141,6 +161,7 @@ struct PoolPlan {
     int64_t gscratch_entries;
     int64_t hscratch_entries;
     int grid, block;
+    int cta_grid;  // resident CTAs of the cooperative passes
 };
 
 rchol_status alloc_work(rchol_ctx* ctx, const PoolPlan& pp) {
@@ -152,7 +173,7 @@ rchol_status alloc_work(rchol_ctx* ctx, const PoolPlan& pp) {
     w.pool_cap = pp.pool_cap;
     w.gscratch_entries = pp.gscratch_entries;
     w.hscratch_entries = pp.hscratch_entries;
-    const int64_t warps = (int64_t)pp.grid * (pp.block / 32);
+    const int64_t slabs = std::max<int64_t>((int64_t)pp.grid * (pp.block / 32), pp.cta_grid);
     CK(dalloc(&w.lcolptr, (int64_t)n + 1), "alloc lcolptr");
     CK(dalloc(&w.lrow, w.lnnz), "alloc lrow");
     CK(dalloc(&w.lval, w.lnnz), "alloc lval");
@@ -172,7 +193,7 @@ rchol_status alloc_work(rchol_ctx* ctx, const PoolPlan& pp) {
     CK(dalloc(&w.hcols, rchol::kHugeColCap + 1), "alloc long-column list");
     CK(dalloc(&w.diag, n), "alloc diag");
     CK(dalloc(&w.level, n), "alloc levels");
-    CK(cudaMalloc((void**)&w.gscratch, (size_t)warps * (size_t)w.gscratch_entries * rchol::kGlobalSlabBytes),
+    CK(cudaMalloc((void**)&w.gscratch, (size_t)slabs * (size_t)w.gscratch_entries * rchol::kGlobalSlabBytes),
        "alloc slab scratch");
     {
         const size_t slab = (size_t)w.hscratch_entries * rchol::kGlobalSlabBytes;
@@ -684,6 +705,10 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     int grid = max_grid;
     if (o.num_blocks > 0) grid = std::max(1, std::min(max_grid, (o.num_blocks + o.warps_per_block - 1) / o.warps_per_block));
 
+    const int max_cta = rchol::factor_cta_grid(ctx->device);
+    if (max_cta <= 0) return fail(ctx, RCHOL_ERR_CUDA, "factor kernel does not fit on the device");
+    const int cta_grid = o.num_blocks > 0 ? std::max(1, std::min(max_cta, o.num_blocks / 8)) : max_cta;
+
     if (!ctx->w_ready) {
         int64_t lnnz = 0;
         rchol_status s = lower_nnz(ctx, &lnnz);
@@ -692,13 +717,14 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
         PoolPlan pp;
         pp.c0 = o.bucket_cap;
         pp.nchunks = (int32_t)std::min<int64_t>(INT32_MAX / 64, std::max<int64_t>(4096, lnnz / 16 + ctx->A.n / 8));
-        pp.pool_cap = (int64_t)(o.pool_mult * (double)lnnz) + ctx->A.n + (int64_t)max_grid * (block / 32) * 1024;
+        pp.pool_cap = (int64_t)(o.pool_mult * (double)lnnz) + ctx->A.n + ((int64_t)max_grid * (block / 32) + 2 * max_cta) * 1024;
         // per-warp scratch up to 4096 entries; larger gathers share nhuge slabs
         const int64_t want = std::max<int64_t>(1024, pow2_ge(4 * (int64_t)ctx->max_lower));
         pp.gscratch_entries = std::min<int64_t>(want, 4096);
         pp.hscratch_entries = want;
         pp.grid = max_grid;
         pp.block = block;
+        pp.cta_grid = max_cta;
         s = alloc_work(ctx, pp);
         if (s != RCHOL_OK) return s;
         ctx->w_ready = true;
@@ -724,6 +750,8 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
         fl.timeout_s = o.timeout_s;
         fl.tail = std::min<int32_t>(std::max(0, o.tail_vertices), ctx->A.n);
         fl.gsize = ctx->gsize;
+        fl.cta = cta_vertices(ctx->A.n, w.lnnz);
+        fl.cta_grid = cta_grid;
         CK(rchol::launch_factor(w, fl, ctx->stream), "factor launch");
         CK(cudaEventRecord(ev[2], ctx->stream), "record");
         CK(cudaMemcpyAsync(counters, w.counters, sizeof(counters), cudaMemcpyDeviceToHost, ctx->stream), "counters");
@@ -736,7 +764,7 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
             return fail(ctx, st == rchol::kDevCapacity ? RCHOL_ERR_CAPACITY : RCHOL_ERR_INVALID,
                         "factor: device status " + std::to_string(st));
         // grow the pool that ran out and retry from scratch
-        PoolPlan pp{w.c0, w.nchunks, w.pool_cap, w.gscratch_entries, w.hscratch_entries, max_grid, block};
+        PoolPlan pp{w.c0, w.nchunks, w.pool_cap, w.gscratch_entries, w.hscratch_entries, max_grid, block, max_cta};
         if (counters[2] >= w.nchunks) pp.nchunks = (int32_t)std::min<int64_t>(INT32_MAX / 64, 2ll * w.nchunks + 1024);
         if ((int64_t)c64[0] > w.pool_cap) pp.pool_cap = 2 * w.pool_cap;
         if ((int64_t)counters[6] > w.hscratch_entries) pp.hscratch_entries = pow2_ge(2 * (int64_t)counters[6]);
@@ -761,8 +789,8 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
                                            o.exact_bwd_levels != 0, o.bwd_head != 0, o.timeout_s, ctx->scratch,
                                            f->F, ctx->stream);
     if (e != cudaSuccess) {
-        free_factor(f->F);
-        delete f;
+        drop_factor(ctx, f);
+        if (e == cudaErrorLaunchTimeout) return fail(ctx, RCHOL_ERR_TIMEOUT, "assembly: a device wait timed out");
         return cuda_fail(ctx, e, "assemble");
     }
     CK(cudaEventRecord(ev[3], ctx->stream), "record");
@@ -770,8 +798,7 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     int32_t sort_status = 0;
     CK(cudaMemcpy(&sort_status, w.counters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost), "status");
     if (sort_status != 0) {
-        free_factor(f->F);
-        delete f;
+        drop_factor(ctx, f);
         return fail(ctx, RCHOL_ERR_CAPACITY, "assembly: row sort scratch too small");
     }
     cudaEventElapsedTime(&info.ms_setup, ev[0], ev[1]);
@@ -916,8 +943,8 @@ rchol_status factor_from_host_csc(rchol_ctx* ctx, int32_t n, const std::vector<i
     }
     cudaFree(dlev);
     if (e != cudaSuccess) {
-        free_factor(F);
-        delete f;
+        drop_factor(ctx, f);
+        if (e == cudaErrorLaunchTimeout) return fail(ctx, RCHOL_ERR_TIMEOUT, "schedule: a device wait timed out");
         return cuda_fail(ctx, e, "upload factor");
     }
     std::memset(&f->info, 0, sizeof(f->info));

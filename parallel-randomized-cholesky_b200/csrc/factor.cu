@@ -15,6 +15,7 @@
 //     first chunk per column plus 64-entry overflow chunks linked lock-free.
 // FP64 arithmetic uses explicitly rounded intrinsics (no contraction), which
 // makes the factor bit-identical to the CPU oracle's ORC_MODE_B200.
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 
@@ -31,7 +32,7 @@ constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 constexpr int kSlabBytesPerEntry = 32;     // 8 (a_val) + 8 (b_val) + 8 (b_aux) + 4 + 4
 
 enum Counter { kQHead = 0, kQTail = 1, kChunkCursor = 2, kStatus = 3, kAbort = 4, kBigCount = 5,
-               kMaxGather = 6, kOverflowFills = 7, kDone = 8, kTailTicket = 9 };
+               kMaxGather = 6, kOverflowFills = 7, kDone = 8, kMidTicket = 9, kTailTicket = 10 };
 
 __device__ __forceinline__ int pow2_at_least(int x) {
     int p = 1;
@@ -87,7 +88,7 @@ __device__ void sort_row_value(int32_t* row, double* val, int P, int lane) {
                     int32_t ri = row[i], rl = row[l];
                     unsigned long long vi = (unsigned long long)__double_as_longlong(val[i]);
                     unsigned long long vl = (unsigned long long)__double_as_longlong(val[l]);
-                    bool gt = (ri > rl) || (ri == rl && vi > vl);
+                    bool gt = (ri > rl) | ((ri == rl) & (vi > vl));
                     bool asc = (i & k) == 0;
                     if (gt == asc) {
                         row[i] = rl;
@@ -111,7 +112,7 @@ __device__ void sort_value_row(double* val, int32_t* row, long long* aux, int P,
                 if (l > i) {
                     double vi = val[i], vl = val[l];
                     int32_t ri = row[i], rl = row[l];
-                    bool gt = (vi > vl) || (vi == vl && ri > rl);
+                    bool gt = (vi > vl) | ((vi == vl) & (ri > rl));
                     bool asc = (i & k) == 0;
                     if (gt == asc) {
                         val[i] = vl;
@@ -326,9 +327,8 @@ struct FactorArgs {
     int smem_slab;
     int smem_region;  // bytes of shared memory per warp (slab, or radix histogram + CDF index)
     unsigned long long timeout_ns;
-    int32_t tail;     // vertices >= tail are left to factor_tail_kernel (n: none)
+    int32_t tail;     // vertices >= tail are left to factor_cta_kernel (n: none)
     int32_t* gsize;   // gathered entries of each vertex (null: not recorded)
-    int32_t tail_cdf_cap;  // prefix sums the tail kernel keeps in shared memory
 };
 
 __device__ __forceinline__ bool aborted(const FactorArgs& a) { return ld_relaxed(a.counters + kAbort) != 0; }
@@ -340,8 +340,13 @@ __device__ __forceinline__ void fail(const FactorArgs& a, int code) {
 
 // Append one fill edge (row > col) to column col's bucket.  Returns false on
 // pool exhaustion.  Chunks are linked with CAS, so no thread ever waits.
-__device__ bool append_fill(const FactorArgs& a, int32_t col, int32_t row, double v) {
-    int s = atomicAdd(a.fcnt + col, 1);
+__device__ bool store_fill(const FactorArgs& a, int32_t col, int32_t row, double v, int s);
+__device__ __forceinline__ bool append_fill(const FactorArgs& a, int32_t col, int32_t row, double v) {
+    return store_fill(a, col, row, v, atomicAdd(a.fcnt + col, 1));
+}
+
+// Fill number s of column col (reserved by the atomic add on its count).
+__device__ bool store_fill(const FactorArgs& a, int32_t col, int32_t row, double v, int s) {
     if (s < a.c0) {
         size_t o = (size_t)col * (size_t)a.c0 + (size_t)s;
         a.brow[o] = row;
@@ -420,14 +425,16 @@ __device__ __forceinline__ bool pool_take(const FactorArgs& a, int m, int lane, 
     return true;
 }
 
-__device__ __forceinline__ bool row_value_gt(int32_t r1, unsigned long long v1, int32_t r2, unsigned long long v2) {
-    return (r1 > r2) || (r1 == r2 && v1 > v2);
-}
+// The release of the cooperative passes: no queue, a CTA waits on the counter
+// itself.  The caller's fence orders the column's writes before it.
+__device__ __forceinline__ void release_row(const FactorArgs& a, int32_t r, int mult) { atomicAdd(a.dep + r, -mult); }
 
 // Elimination of a vertex whose gathered list fits one warp (at most 32
 // entries, all fills in the first bucket chunk): one entry per lane; sorts,
 // merge, compaction, scan and CDF search as warp shuffles.  Same arithmetic
 // in the same order as the slab path (and the oracle), so the bits agree.
+// QUEUE: released neighbours go to `next` and the ready queue.
+template <bool QUEUE>
 __device__ bool eliminate_small(const FactorArgs& a, int32_t k, int total, int32_t brow_l, double bval_l, int lvl,
                                 int lane, int64_t& pool_cur, int64_t& pool_end, long long& fills, int32_t& next) {
     // all `total` entries sit in the bucket, entry `lane` in this lane
@@ -445,11 +452,11 @@ __device__ bool eliminate_small(const FactorArgs& a, int32_t k, int total, int32
             const int32_t r2 = __shfl_xor_sync(kFull, row, j);
             const unsigned long long v2 = __shfl_xor_sync(kFull, vb, j);
             const bool keep_min = ((lane & j) == 0) == ((lane & kk) == 0);
-            const bool take = keep_min ? row_value_gt(row, vb, r2, v2) : row_value_gt(r2, v2, row, vb);
-            if (take) {
-                row = r2;
-                vb = v2;
-            }
+            // no short circuits: as branches the two networks took twice as long
+            const bool gt = (row > r2) | ((row == r2) & (vb > v2));
+            const bool take = keep_min == gt;  // fully equal keys may trade places
+            row = take ? r2 : row;
+            vb = take ? v2 : vb;
         }
     }
     // merge equal rows: the head of each run sums its run left to right
@@ -478,33 +485,33 @@ __device__ bool eliminate_small(const FactorArgs& a, int32_t k, int total, int32
     // merged entries in row order, entry `lane` in this lane
     int32_t orow = __shfl_sync(kFull, row, src);
     int ocnt = __shfl_sync(kFull, cnt, src);
-    double mval = __shfl_sync(kFull, acc, src);
+    unsigned long long mbits = (unsigned long long)__double_as_longlong(__shfl_sync(kFull, acc, src));
     if (lane >= m) {
         orow = INT_MAX;
         ocnt = 0;
-        mval = __longlong_as_double((long long)kInfBits);
+        mbits = ~0ull;
     }
     int pos = lane;  // position in row order
     // sort by (value, row) carrying the row-order position.  Rows are unique
     // and ascend with the position, so ties in value break on the position
-    // exactly as on the row (padding, all +inf, sorts last in any order);
+    // exactly as on the row (nonnegative values order as their bits; padding,
+    // all ones, sorts last);
     // the row and multiplicity are fetched by position afterwards, which
     // keeps two shuffles per stage off the shared-memory/shuffle pipe.
 #pragma unroll
     for (int kk = 2; kk <= 32; kk <<= 1) {
 #pragma unroll
         for (int j = kk >> 1; j > 0; j >>= 1) {
-            const double v2 = __shfl_xor_sync(kFull, mval, j);
+            const unsigned long long v2 = __shfl_xor_sync(kFull, mbits, j);
             const int p2 = __shfl_xor_sync(kFull, pos, j);
             const bool keep_min = ((lane & j) == 0) == ((lane & kk) == 0);
-            const bool self_gt = (mval > v2) || (mval == v2 && pos > p2);
-            const bool other_gt = (v2 > mval) || (v2 == mval && p2 > pos);
-            if (keep_min ? self_gt : other_gt) {
-                mval = v2;
-                pos = p2;
-            }
+            const bool gt = (mbits > v2) | ((mbits == v2) & (pos > p2));
+            const bool take = keep_min == gt;
+            mbits = take ? v2 : mbits;
+            pos = take ? p2 : pos;
         }
     }
+    const double mval = __longlong_as_double((long long)mbits);
     const int32_t mrow = __shfl_sync(kFull, orow, pos);
     const int mcnt = __shfl_sync(kFull, ocnt, pos);
     // inclusive prefix sum (one 32-wide Kogge-Stone chunk)
@@ -558,9 +565,14 @@ __device__ bool eliminate_small(const FactorArgs& a, int32_t k, int total, int32
         return false;
     }
     const int lk = lvl + 1;
+    if (!QUEUE && lane < m) atomicMax(a.level + mrow, lk);
     __threadfence();
     __syncwarp();
-    release_chunk(a, lk, lane, lane < m, mrow, mcnt, next);
+    if (QUEUE) {
+        release_chunk(a, lk, lane, lane < m, mrow, mcnt, next);
+    } else if (lane < m) {
+        release_row(a, mrow, mcnt);
+    }
     __syncwarp();
     return true;
 }
@@ -641,7 +653,7 @@ __device__ bool eliminate(const FactorArgs& a, int32_t k, Slab sm, unsigned char
     if (total > max_gather) max_gather = total;
     if (a.gsize && lane == 0) a.gsize[k] = total;
     if (no == 0 && nf <= a.c0 && total <= kWarp)  // every entry is in the bucket
-        return eliminate_small(a, k, total, brow_l, bval_l, lvl, lane, pool_cur, pool_end, fills, next);
+        return eliminate_small<true>(a, k, total, brow_l, bval_l, lvl, lane, pool_cur, pool_end, fills, next);
     if (total <= a.smem_slab)
         return eliminate_slab<false>(a, k, nf, o0, no, lvl, sm, wsm, lane, pool_cur, pool_end, fills, next);
     if (lane == 0) atomicAdd(a.counters + kBigCount, 1);
@@ -939,39 +951,163 @@ __global__ void __launch_bounds__(256, 3) factor_kernel(FactorArgs a) {
     if (lane == 0 && fills) atomicAdd(a.pool_cursor + 1, (unsigned long long)fills);
 }
 
-// ---- cooperative elimination of the tail -----------------------------------
-// The last vertices of a power-law graph (hubs and the dense core) depend
-// on one another in long chains and gather thousands of entries each; a
-// warp per vertex leaves the rest of the GPU idle while it sorts.  Vertices
-// >= tail are therefore eliminated after factor_kernel by nhuge CTAs of
-// kTailThreads threads, a whole CTA per vertex.  A CTA claims the next
-// vertex in index order and waits on its dependency counter (every
-// dependency has a smaller index, hence was claimed earlier by a running
-// CTA), then keeps the counters as factor_kernel does: +1 per fill row,
-// -multiplicity per neighbour once the column is written.  The steps
-// and their rounding are those of eliminate_slab<true> -- the same radix
-// orders, duplicate runs added in sorted order, 32-wide Kogge-Stone chunks
-// with the carry chained in chunk order, the same sampling search -- so the
-// factor is bit-identical to the warp path's (and the oracle's).
+// ---- cooperative elimination: a CTA per vertex -------------------------------
+// The vertices eliminated last form the long dependency chains of the
+// elimination (levels of a few dozen vertices) and gather the longest lists,
+// so a warp per vertex leaves most of the GPU idle while single warps sort.
+// Vertices >= cta_begin are therefore eliminated after factor_kernel, a
+// whole CTA per vertex.  A CTA claims the next vertex in index order and
+// waits on its dependency counter (every dependency has a smaller index, hence
+// was claimed earlier by a running CTA), then keeps the counters as
+// factor_kernel does: +1 per fill row, -multiplicity per neighbour once the
+// column is written.
+//
+// A list of at most 32 entries is one warp's (eliminate_small).  Up to NT * E
+// entries are sorted in blocks of 32 by register bitonic networks, then merged
+// up to 8 blocks at a time by ranks: every entry finds its rank among the other
+// blocks by binary searches in shared memory, all searches of an entry in
+// flight together, and moves once per round.  Longer lists take CTA-wide radix passes
+// over a slab in global memory.  The steps and their rounding are those of
+// eliminate_slab -- the same unique orders, duplicate runs added in sorted
+// order, 32-wide Kogge-Stone chunks with the carry chained in chunk order, the
+// same sampling search -- so the factor is bit-identical to the warp path's
+// (and the oracle's).
+//
+// What bounds it is one vertex's latency along the chain: for a list of 46 / 92 /
+// 168 / 314 entries 12.4 / 15.8 / 19.9 / 33.6 k cycles from claim to release,
+// a quarter of it the sampling with its reservation round trip (a warp took
+// about 35 / 60 k cycles for lists of 33-64 / 65-128).  Factor time, a warp per
+// vertex -> this: 7-point 128^3 13.3 -> 9.5 ms, 27-point 72x70x67 106 -> 20.7 ms,
+// 100 k-vertex Chung-Lu 63 -> 23.4 ms with a tail of 1500, 198 -> 55 ms without.
+//
+// Two instances: <256, 4>, several CTAs per SM, for the late vertices of any
+// matrix (cta_vertices in capi.cpp says how many), and <1024, 4>, one CTA per
+// SM, for the hubs and the dense core of power-law graphs (the tail_vertices
+// option).
 
-constexpr int kTailThreads = 1024;
-constexpr int kTailWarps = kTailThreads / kWarp;
-// shared memory of the tail kernel: per-warp digit histograms, 256 totals
-// (+ a flag), warp offsets, padded to an even word count; then a copy of up
-// to kTailCdfCap prefix sums for the sampling searches
-constexpr int kTailIntWords = kTailWarps * 256 + 260 + 36;
-constexpr int kTailCdfCap = 20480;
-static_assert(kTailIntWords % 2 == 0, "the prefix-sum copy must be 8-byte aligned");
+// Sorts n keys (tag, value bits), thread t holding positions t, t + NT, ...
+// (positions past n hold the greatest key): by (tag, value bits), or, BYVAL, by
+// value bits with ties in entry order (the tag must be the position on entry).
+// The sorted keys end in the registers by position and in one of the buffer
+// pairs (x0, r0), (x1, r1), which is returned (0 or 1).  Ends with a barrier.
+// The comparisons are written without short circuits: as branches they took
+// three times as long (a stage of a 32-key network 240 cycles instead of 80).
+template <int NT, int EE, bool BYVAL>
+__device__ __forceinline__ int cta_sort(int32_t (&t)[EE], unsigned long long (&v)[EE], int n, unsigned long long* x0,
+                                        unsigned long long* x1, int32_t* r0, int32_t* r1) {
+    const int tid = threadIdx.x, lane = tid & 31;
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        const int i = e * NT + tid;
+        if (i - lane < n) {
+#pragma unroll
+            for (int kk = 2; kk <= kWarp; kk <<= 1) {
+#pragma unroll
+                for (int j = kk >> 1; j > 0; j >>= 1) {
+                    const int32_t t2 = __shfl_xor_sync(kFull, t[e], j);
+                    const unsigned long long v2 = __shfl_xor_sync(kFull, v[e], j);
+                    const bool lower = ((lane & j) == 0) == ((lane & kk) == 0);
+                    const bool gt = BYVAL ? (v[e] > v2) | ((v[e] == v2) & (t[e] > t2))
+                                          : (t[e] > t2) | ((t[e] == t2) & (v[e] > v2));
+                    const bool take = lower == gt;  // fully equal keys may trade places
+                    t[e] = take ? t2 : t[e];
+                    v[e] = take ? v2 : v[e];
+                }
+            }
+            if (i < n) {
+                x0[i] = v[e];
+                r0[i] = t[e];
+            }
+        }
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int len = kWarp; len < n; len <<= 3) {
+        const unsigned long long* xs = cur ? x1 : x0;
+        const int32_t* rs = cur ? r1 : r0;
+        unsigned long long* xd = cur ? x0 : x1;
+        int32_t* rd = cur ? r0 : r1;
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int i = e * NT + tid;
+            if (i - lane >= n) continue;
+            const int base = i & ~(8 * len - 1);
+            const int own = (i - base) / len;
+            int rank = i - own * len;
+            // entries before this one in each of the other blocks (equal keys
+            // of earlier blocks come first): 4 searches in lockstep, so that
+            // their loads overlap
+            for (int b0 = 0; b0 < 8 && base + b0 * len < n; b0 += 4) {
+                int at[4], end[4];
+                unsigned long long lim[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int st = base + (b0 + q) * len;
+                    at[q] = st - 1;
+                    end[q] = b0 + q == own ? -1 : min(st + len, n);
+                    lim[q] = v[e] + (b0 + q < own ? 1 : 0);
+                }
+                for (int step = len; step > 0; step >>= 1) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int to = at[q] + step;
+                        const bool in = to < end[q];
+                        const int probe = in ? to : 0;
+                        bool before = xs[probe] < lim[q];
+                        if (!BYVAL) {
+                            const int32_t tp = rs[probe];
+                            before = (tp < t[e]) | ((tp == t[e]) & before);
+                        }
+                        at[q] = (in & before) ? to : at[q];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) rank += at[q] + 1 - (base + (b0 + q) * len);
+            }
+            if (i < n) {
+                xd[rank] = v[e];
+                rd[rank] = t[e];
+            }
+        }
+        __syncthreads();
+        cur ^= 1;
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int i = e * NT + tid;
+            if (i < n) {
+                v[e] = (cur ? x1 : x0)[i];
+                t[e] = (cur ? r1 : r0)[i];
+            }
+        }
+    }
+    return cur;
+}
+
+// The partner sampled for value-order position i: the first j > i with
+// C_j - C_i >= u * (S - C_i), C the prefix sums.
+__device__ __forceinline__ int sample_partner(const FactorArgs& a, int32_t k, int i, int m, const double* C,
+                                              double rem_i) {
+    const double ci = C[i];
+    const double target = __dmul_rn(sample_uniform(a.seed, k, i), rem_i);
+    int lo = i + 1, hi = m;
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if (__dsub_rn(C[mid], ci) < target) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < m ? lo : m - 1;
+}
 
 // One stable CTA pass of (row, val[, aux]) by digit d: warp w takes a
 // contiguous tile (a multiple of 32 entries), counts, and scatters it in
 // order through digit-major, warp-minor offsets.  Returns false when one
 // digit holds all n entries (nothing would move; nothing is written).
-template <bool VR, bool AUX>
-__device__ bool tail_radix_pass(const int32_t* row, const double* val, const long long* aux, int32_t* orow,
-                                double* oval, long long* oaux, int n, int d, int* hist, int* tot) {
+template <int NT, bool VR, bool AUX>
+__device__ bool cta_radix_pass(const int32_t* row, const double* val, const long long* aux, int32_t* orow,
+                               double* oval, long long* oaux, int n, int d, int* hist, int* tot) {
+    constexpr int NW = NT / kWarp;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int tile = ((n + kTailWarps - 1) / kTailWarps + 31) & ~31;
+    const int tile = ((n + NW - 1) / NW + 31) & ~31;
     const int t0 = min(n, w * tile), t1 = min(n, t0 + tile);
     int* h = hist + w * 256;
     for (int i = lane; i < 256; i += kWarp) h[i] = 0;
@@ -990,7 +1126,7 @@ __device__ bool tail_radix_pass(const int32_t* row, const double* val, const lon
     __syncthreads();
     if (threadIdx.x < 256) {
         int c = 0;
-        for (int q = 0; q < kTailWarps; ++q) c += hist[q * 256 + threadIdx.x];
+        for (int q = 0; q < NW; ++q) c += hist[q * 256 + threadIdx.x];
         tot[threadIdx.x] = c;
     }
     __syncthreads();
@@ -1022,7 +1158,7 @@ __device__ bool tail_radix_pass(const int32_t* row, const double* val, const lon
     const bool skip = tot[256] != 0;
     if (!skip && threadIdx.x < 256) {
         int run = tot[threadIdx.x];
-        for (int q = 0; q < kTailWarps; ++q) {
+        for (int q = 0; q < NW; ++q) {
             const int c = hist[q * 256 + threadIdx.x];
             hist[q * 256 + threadIdx.x] = run;
             run += c;
@@ -1068,14 +1204,14 @@ __device__ bool tail_radix_pass(const int32_t* row, const double* val, const lon
     return true;
 }
 
-template <bool VR, bool AUX>
-__device__ void tail_radix_sort(int32_t* r_out, double* v_out, long long* x_out, int32_t* r_tmp, double* v_tmp,
-                                long long* x_tmp, int n, int dlo, int dhi, int* hist, int* tot) {
+template <int NT, bool VR, bool AUX>
+__device__ void cta_radix_sort(int32_t* r_out, double* v_out, long long* x_out, int32_t* r_tmp, double* v_tmp,
+                               long long* x_tmp, int n, int dlo, int dhi, int* hist, int* tot) {
     int32_t *r0 = r_out, *r1 = r_tmp;
     double *v0 = v_out, *v1 = v_tmp;
     long long *x0 = x_out, *x1 = x_tmp;
     for (int d = dlo; d < dhi; ++d) {
-        if (!tail_radix_pass<VR, AUX>(r0, v0, x0, r1, v1, x1, n, d, hist, tot)) continue;
+        if (!cta_radix_pass<NT, VR, AUX>(r0, v0, x0, r1, v1, x1, n, d, hist, tot)) continue;
         int32_t* tr = r0;
         r0 = r1;
         r1 = tr;
@@ -1087,7 +1223,7 @@ __device__ void tail_radix_sort(int32_t* r_out, double* v_out, long long* x_out,
         x1 = tx;
     }
     if (r0 != r_out) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        for (int i = threadIdx.x; i < n; i += NT) {
             r_out[i] = r0[i];
             v_out[i] = v0[i];
             if (AUX) x_out[i] = x0[i];
@@ -1096,59 +1232,281 @@ __device__ void tail_radix_sort(int32_t* r_out, double* v_out, long long* x_out,
     }
 }
 
-// Exclusive count of the flagged entries before each warp's tile, for an
-// order-preserving compaction (warp w holds the tile as in the radix passes).
-__device__ __forceinline__ int tail_tile_offset(int count, int* scan) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) scan[w] = count;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int q = 0; q < kTailWarps; ++q) {
-            const int c = scan[q];
-            scan[q] = run;
-            run += c;
+// Shared memory of the cooperative kernel: the register path's arrays (32 B
+// per entry: two value and three tag buffers and the multiplicities), or the
+// radix path's per-warp digit counts and totals followed by as many prefix
+// sums as fit.
+template <int NT, int E>
+struct CtaPlan {
+    static constexpr int kWarps = NT / kWarp;
+    static constexpr int kCap = NT * E;
+    static constexpr int kRadixWords = kWarps * 256 + 260;
+    static constexpr int kBytes = 32 * kCap > 4 * kRadixWords + 8192 ? 32 * kCap : 4 * kRadixWords + 8192;
+    static constexpr int kCdf = (kBytes - 4 * kRadixWords) / 8;
+    static_assert((4 * kRadixWords) % 8 == 0, "the prefix sums must be 8-byte aligned");
+};
+
+// What a CTA found for its vertex, and its shared state.
+struct CtaVertex {
+    int32_t k;
+    int nf, n0;    // fills in the column's bucket and chunks; those in the bucket
+    int o0, no;    // originals that did not fit the bucket: lrow[o0 .. o0 + no)
+    int total, lk;
+    int chunk;     // first overflow chunk
+    int32_t brow;  // bucket slot threadIdx.x
+    double bval;
+};
+
+// Elimination of a vertex of at most NT * EE entries in shared memory.
+// Returns false if the kernel must stop.
+template <int NT, int EE>
+__device__ __forceinline__ bool cta_eliminate(const FactorArgs& a, const CtaVertex& V, unsigned char* smem, int cap,
+                                              int* scan, double* ctot, int64_t* sh_base, int64_t& pool_cur,
+                                              int64_t& pool_end, long long& fills) {
+    constexpr int NW = NT / kWarp;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int total = V.total;
+    unsigned long long* x0 = reinterpret_cast<unsigned long long*>(smem);
+    unsigned long long* x1 = x0 + cap;
+    int32_t* r0 = reinterpret_cast<int32_t*>(x1 + cap);
+    int32_t* r1 = r0 + cap;
+    int32_t* r2 = r1 + cap;
+    int32_t* mult = r2 + cap;
+    const size_t bo = (size_t)V.k * (size_t)a.c0;
+    // ---- gather: the bucket's first NT slots are in registers
+    int32_t tg[EE];
+    unsigned long long vb[EE];
+    if (V.nf <= a.c0) {
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int i = e * NT + tid;
+            double v = 0.0;
+            tg[e] = INT_MAX;
+            if (e == 0 && i < V.n0) {
+                tg[e] = V.brow;
+                v = V.bval;
+            } else if (i < V.n0) {
+                tg[e] = __ldcg(a.brow + bo + i);
+                v = __ldcg(a.bval + bo + i);
+            } else if (i < total) {
+                tg[e] = a.lrow[V.o0 + i - V.n0];
+                v = a.lval[V.o0 + i - V.n0];
+            }
+            vb[e] = i < total ? (unsigned long long)__double_as_longlong(v) : ~0ull >> 1;
         }
-        scan[kTailWarps] = run;
+    } else {
+        double* g = reinterpret_cast<double*>(x1);
+        for (int i = tid; i < V.n0; i += NT) {
+            r1[i] = i == tid ? V.brow : __ldcg(a.brow + bo + i);
+            g[i] = i == tid ? V.bval : __ldcg(a.bval + bo + i);
+        }
+        for (int i = tid; i < V.no; i += NT) {
+            r1[V.nf + i] = a.lrow[V.o0 + i];
+            g[V.nf + i] = a.lval[V.o0 + i];
+        }
+        int rem = V.nf - V.n0, pos = V.n0, chunk = V.chunk;
+        for (int lvl = 0; rem > 0; ++lvl) {
+            if (chunk < 0 || chunk > a.nchunks - (1 << lvl)) {  // the same for every thread
+                if (tid == 0) fail(a, kDevBadInput);
+                return false;
+            }
+            const int cnt = min(rem, kChunk << lvl);
+            const int link = rem > cnt ? ld_relaxed(a.cnext + chunk) : -1;
+            for (int i = tid; i < cnt; i += NT) {
+                r1[pos + i] = __ldcg(a.crow + (size_t)chunk * kChunk + i);
+                g[pos + i] = __ldcg(a.cval + (size_t)chunk * kChunk + i);
+            }
+            pos += cnt;
+            rem -= cnt;
+            chunk = link;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int i = e * NT + tid;
+            tg[e] = i < total ? r1[i] : INT_MAX;
+            vb[e] = i < total ? x1[i] : ~0ull >> 1;
+        }
+    }
+    // ---- sort by (row, value bits); merge duplicate rows in that order
+    const int c1 = cta_sort<NT, EE, false>(tg, vb, total, x0, x1, r0, r1);
+    unsigned long long* fx = c1 ? x1 : x0;  // the sorted list
+    int32_t* fr = c1 ? r1 : r0;
+    unsigned long long* ox = c1 ? x0 : x1;  // the merged one
+    int32_t* orow = c1 ? r0 : r1;
+    bool head[EE];
+    int pre[EE];
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        const int i = e * NT + tid;
+        head[e] = i < total && (i == 0 || fr[i - 1] != tg[e]);
+        const unsigned bal = __ballot_sync(kFull, head[e]);
+        pre[e] = __popc(bal & lt);
+        if (lane == 0) scan[e * NW + w] = __popc(bal);
     }
     __syncthreads();
-    return scan[w];
+    // every warp scans the NW * EE counts for itself
+    int m = 0;
+#pragma unroll
+    for (int q0 = 0; q0 < NW * EE; q0 += kWarp) {
+        const int c = q0 + lane < NW * EE ? scan[q0 + lane] : 0;
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int before = __shfl_sync(kFull, incl - c, (e * NW + w) & 31);
+            if (e * NW + w >= q0 && e * NW + w < q0 + kWarp) pre[e] += m + before;
+        }
+        m += __shfl_sync(kFull, incl, kWarp - 1);
+    }
+    if (w == 0) {
+        int64_t base = -1;
+        if (!pool_take(a, m, lane, pool_cur, pool_end, base)) base = -1;
+        if (lane == 0) *sh_base = base;
+    }
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        if (!head[e]) continue;
+        double acc = __longlong_as_double((long long)vb[e]);
+        int cnt = 1;
+        for (int j = e * NT + tid + 1; j < total && fr[j] == tg[e]; ++j) {
+            acc = __dadd_rn(acc, __longlong_as_double((long long)fx[j]));
+            ++cnt;
+        }
+        ox[pre[e]] = (unsigned long long)__double_as_longlong(acc);
+        orow[pre[e]] = tg[e];
+        mult[pre[e]] = cnt;
+    }
+    __syncthreads();
+    const int64_t pbase = *sh_base;
+    if (pbase < 0) {
+        if (tid == 0) fail(a, kDevCapacity);
+        return false;
+    }
+    // ---- sort by (value, row): rows ascend with the row-order position
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        const int i = e * NT + tid;
+        tg[e] = i;
+        vb[e] = i < m ? ox[i] : ~0ull >> 1;
+    }
+    const int c2 = cta_sort<NT, EE, true>(tg, vb, m, fx, ox, fr, r2);
+    double* C = reinterpret_cast<double*>(c2 ? fx : ox);  // the buffers the sort left free
+    int32_t* rowv = c2 ? fr : r2;
+    // ---- prefix sums: 32-wide Kogge-Stone chunks, the carries chained in
+    // chunk order, as the warp path carries them
+    double f[EE];
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        const int i = e * NT + tid;
+        f[e] = 0.0;
+        if (i - lane < m) {
+            double v = i < m ? __longlong_as_double((long long)vb[e]) : 0.0;
+#pragma unroll
+            for (int off = 1; off < kWarp; off <<= 1) {
+                const double t = __shfl_up_sync(kFull, v, off);
+                if (lane >= off) v = __dadd_rn(v, t);
+            }
+            f[e] = v;
+            if (lane == kWarp - 1) ctot[e * NW + w] = v;
+        }
+        if (i < m) rowv[i] = orow[tg[e]];
+    }
+    __syncthreads();
+    {
+        // every warp chains the chunk totals before its own chunks
+        double carry = 0.0;
+        int q = 0;
+#pragma unroll
+        for (int e = 0; e < EE; ++e) {
+            const int i = e * NT + tid;
+            if (i - lane >= m) continue;
+            for (; q < e * NW + w; ++q) carry = q == 0 ? ctot[0] : __dadd_rn(carry, ctot[q]);
+            if (i < m) {
+                if (i >= kWarp) f[e] = __dadd_rn(carry, f[e]);
+                C[i] = f[e];
+            }
+        }
+    }
+    __syncthreads();
+    const double S = C[m - 1];
+    // ---- clique sampling, L column k (row order) and D_k
+    if (tid == 0) {
+        a.diag[V.k] = S;
+        a.pstart[V.k] = pbase;
+        a.pcnt[V.k] = m;
+    }
+    bool ok = true;
+#pragma unroll
+    for (int e = 0; e < EE; ++e) {
+        const int i = e * NT + tid;
+        if (i >= m) continue;
+        const double vi = __longlong_as_double((long long)vb[e]);
+        const int32_t r = rowv[i];
+        int32_t grow = 0, gcol = 0;
+        int slot = 0;
+        double rem_i = 0.0;
+        if (i < m - 1) {
+            rem_i = __dsub_rn(S, C[i]);
+            const int32_t rj = rowv[sample_partner(a, V.k, i, m, C, rem_i)];
+            grow = r > rj ? r : rj;
+            gcol = r > rj ? rj : r;
+            slot = atomicAdd(a.fcnt + gcol, 1);  // the rest runs while it is under way
+            atomicAdd(a.dep + grow, 1);
+        }
+        a.prow[pbase + tg[e]] = r;
+        a.pval[pbase + tg[e]] = __ddiv_rn(vi, S);
+        atomicMax(a.level + r, V.lk);
+        if (i < m - 1 && !store_fill(a, gcol, grow, __ddiv_rn(__dmul_rn(vi, rem_i), S), slot)) ok = false;
+    }
+    // fills, pool writes and levels are visible before any neighbour is
+    // released: each neighbour's counter drops by its multiplicity
+    __threadfence();
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) fail(a, kDevCapacity);
+        return false;
+    }
+    for (int i = tid; i < m; i += NT) release_row(a, orow[i], mult[i]);
+    fills += m - 1;
+    return true;
 }
 
-__global__ void __launch_bounds__(kTailThreads, 1) factor_tail_kernel(FactorArgs a) {
+template <int NT, int E>
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 1) factor_cta_kernel(FactorArgs a, int32_t begin, int32_t end,
+                                                                         int ticket) {
+    using Plan = CtaPlan<NT, E>;
+    constexpr int NW = Plan::kWarps;
+    constexpr int kCap = Plan::kCap;
     extern __shared__ __align__(16) unsigned char smem[];
-    int* hist = reinterpret_cast<int*>(smem);      // [kTailWarps][256]
-    int* tot = hist + kTailWarps * 256;            // [257]
-    int* scan = tot + 260;                         // [kTailWarps + 1]
-    __shared__ long long sh_base;
-    __shared__ int sh_stop;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ int scan[NW * E + 2];
+    __shared__ double ctot[kCap / kWarp];
+    __shared__ int64_t sh_base;
+    __shared__ int32_t sh_k, sh_lock;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
     long long fills = 0;
     int max_gather = 0;
-    __shared__ int32_t sh_k;
-    if (threadIdx.x == 0) sh_stop = 0;
-    __syncthreads();
-    // CTA b works in huge slab b (the persistent kernel, which shares them
-    // under locks, has finished)
-    Slab s = make_global_slab(a.hscratch + (size_t)blockIdx.x * (size_t)a.hscratch_entries * kGlobalSlabBytes,
-                              (int)a.hscratch_entries);
-    const unsigned long long t0 = global_timer_ns();
+    int64_t pool_cur = 0, pool_end = 0;  // warp 0's
+    const unsigned long long t_start = global_timer_ns();
     while (true) {
-        // claim the next tail vertex in index order and wait until every
-        // column it depends on is eliminated (all have lower indices, so
-        // they were claimed earlier by running CTAs); the wait is bounded
-        // by time without progress of the eliminated count
-        if (threadIdx.x == 0) {
-            int32_t k = a.tail + atomicAdd(a.counters + kTailTicket, 1);
-            if (k < a.n) {
+        // claim the next vertex in index order and wait until every column
+        // it depends on is eliminated; the wait is bounded by time without
+        // progress of the eliminated count
+        if (tid == 0) {
+            int32_t k = begin + atomicAdd(a.counters + ticket, 1);
+            if (k < end) {
                 unsigned spins = 0;
                 int seen = -1;
-                unsigned long long since = t0;
+                unsigned long long since = t_start;
                 while (ld_acquire(a.dep + k) > 0) {
                     if ((++spins & 63u) == 0) {
                         if (aborted(a)) {
-                            k = a.n;
+                            k = end;
                             break;
                         }
                         const int d = ld_relaxed(a.counters + kDone);
@@ -1158,27 +1516,41 @@ __global__ void __launch_bounds__(kTailThreads, 1) factor_tail_kernel(FactorArgs
                             since = now;
                         } else if (now - since > a.timeout_ns) {
                             fail(a, kDevTimeout);
-                            k = a.n;
+                            k = end;
                             break;
                         }
                     }
                 }
             }
-            sh_k = k;
+            sh_k = k < end ? k : end;
         }
         __syncthreads();
         const int32_t k = sh_k;
-        if (k >= a.n) break;
+        if (k >= end) break;
         __threadfence();
-        const int nf = ld_relaxed(a.fcnt + k);
+        // one round trip: the counts, the level and the bucket's first slots
+        CtaVertex V;
+        V.k = k;
+        const size_t bo = (size_t)k * (size_t)a.c0;
+        V.brow = 0;
+        V.bval = 0.0;
+        if (tid < a.c0) {
+            V.brow = __ldcg(a.brow + bo + tid);
+            V.bval = __ldcg(a.bval + bo + tid);
+        }
+        V.nf = ld_relaxed(a.fcnt + k);
+        V.chunk = ld_relaxed(a.chead + k);
         const int oc0 = a.lcolptr[k];
         const int ocnt = a.lcolptr[k + 1] - oc0;
-        const int o0 = oc0 + min(ocnt, a.c0);
-        const int no = ocnt - min(ocnt, a.c0);
-        const int total = nf + no;
-        if (a.gsize && threadIdx.x == 0) a.gsize[k] = total;
-        if (total == 0) {
-            if (threadIdx.x == 0) {
+        V.lk = ld_relaxed(a.level + k) + 1;  // rows of L column k are at least one level below k
+        V.o0 = oc0 + min(ocnt, a.c0);
+        V.no = ocnt - min(ocnt, a.c0);
+        V.n0 = min(V.nf, a.c0);
+        V.total = V.nf + V.no;
+        const int nf = V.nf, n0 = V.n0, o0 = V.o0, no = V.no, total = V.total, lk = V.lk;
+        if (a.gsize && tid == 0) a.gsize[k] = total;
+        if (total == 0) {  // empty column, D = 0
+            if (tid == 0) {
                 a.diag[k] = 0.0;
                 a.pcnt[k] = 0;
                 a.pstart[k] = 0;
@@ -1188,186 +1560,207 @@ __global__ void __launch_bounds__(kTailThreads, 1) factor_tail_kernel(FactorArgs
             continue;
         }
         if (total > max_gather) max_gather = total;
-        if ((int64_t)total > a.hscratch_entries) {
-            if (threadIdx.x == 0) fail(a, kDevCapacity);
-            break;
-        }
-        // ---- gather: bucket, overflow chunks, originals
-        const int n0 = min(nf, a.c0);
-        for (int t = threadIdx.x; t < n0; t += blockDim.x) {
-            const size_t o = (size_t)k * (size_t)a.c0 + (size_t)t;
-            s.a_row[t] = __ldcg(a.brow + o);
-            s.a_val[t] = __ldcg(a.bval + o);
-        }
-        int rem = nf - n0, pos = n0;
-        int chunk = rem > 0 ? ld_relaxed(a.chead + k) : -1;
-        bool bad = false;
-        for (int lvl = 0; rem > 0; ++lvl) {
-            if (chunk < 0 || chunk > a.nchunks - (1 << lvl)) {
-                bad = true;
+        bool go = true;
+        if (nf <= a.c0 && no == 0 && total <= kWarp) {
+            if (w == 0) {
+                int32_t next = -1;
+                if (lane >= total) V.brow = INT_MAX;
+                go = eliminate_small<false>(a, k, total, V.brow, V.bval, lk - 1, lane, pool_cur, pool_end, fills, next);
+            }
+            if (__syncthreads_or(!go)) break;
+        } else if (total <= NT) {
+            go = cta_eliminate<NT, 1>(a, V, smem, kCap, scan, ctot, &sh_base, pool_cur, pool_end, fills);
+            if (!go) break;
+        } else if (total <= 2 * NT) {
+            go = cta_eliminate<NT, 2>(a, V, smem, kCap, scan, ctot, &sh_base, pool_cur, pool_end, fills);
+            if (!go) break;
+        } else if (total <= kCap) {
+            go = cta_eliminate<NT, E>(a, V, smem, kCap, scan, ctot, &sh_base, pool_cur, pool_end, fills);
+            if (!go) break;
+        } else {
+            int* hist = reinterpret_cast<int*>(smem);  // [NW][256]
+            int* tot = hist + NW * 256;                // [257]
+            int m = 0, lock = -1;
+            bool ok = true;
+            if (tid == 0) {
+                atomicAdd(a.counters + kBigCount, 1);
+                sh_lock = -2;
+                if ((int64_t)total > a.hscratch_entries) fail(a, kDevCapacity);
+            }
+            if ((int64_t)total > a.hscratch_entries) break;
+            Slab s;
+            if ((int64_t)total <= a.gscratch_entries) {
+                s = make_global_slab(a.gscratch + (size_t)blockIdx.x * (size_t)a.gscratch_entries * kGlobalSlabBytes,
+                                     (int)a.gscratch_entries);
+            } else {
+                __syncthreads();
+                if (w == 0) {
+                    const int h = acquire_huge(a, lane);
+                    if (lane == 0) sh_lock = h;
+                }
+                __syncthreads();
+                lock = sh_lock;
+                if (lock < 0) break;
+                s = make_global_slab(a.hscratch + (size_t)lock * (size_t)a.hscratch_entries * kGlobalSlabBytes,
+                                     (int)a.hscratch_entries);
+            }
+            // ---- gather: bucket, overflow chunks, originals
+            for (int t = tid; t < n0; t += NT) {
+                s.a_row[t] = __ldcg(a.brow + bo + t);
+                s.a_val[t] = __ldcg(a.bval + bo + t);
+            }
+            int rem = nf - n0, pos = n0;
+            int chunk = V.chunk;
+            for (int lvl = 0; rem > 0; ++lvl) {
+                if (chunk < 0 || chunk > a.nchunks - (1 << lvl)) {
+                    ok = false;
+                    break;
+                }
+                const int cnt = min(rem, kChunk << lvl);
+                for (int t = tid; t < cnt; t += NT) {
+                    s.a_row[pos + t] = __ldcg(a.crow + (size_t)chunk * kChunk + t);
+                    s.a_val[pos + t] = __ldcg(a.cval + (size_t)chunk * kChunk + t);
+                }
+                pos += cnt;
+                rem -= cnt;
+                if (rem > 0) chunk = ld_relaxed(a.cnext + chunk);
+            }
+            if (!ok) {  // the kernel stops; held slabs are reset with the next factorization's state
+                if (tid == 0) fail(a, kDevBadInput);
                 break;
             }
-            const int cnt = min(rem, kChunk << lvl);
-            for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-                s.a_row[pos + t] = __ldcg(a.crow + (size_t)chunk * kChunk + t);
-                s.a_val[pos + t] = __ldcg(a.cval + (size_t)chunk * kChunk + t);
+            for (int t = tid; t < no; t += NT) {
+                s.a_row[nf + t] = a.lrow[o0 + t];
+                s.a_val[nf + t] = a.lval[o0 + t];
             }
-            pos += cnt;
-            rem -= cnt;
-            if (rem > 0) chunk = ld_relaxed(a.cnext + chunk);
-        }
-        if (bad) {
-            if (threadIdx.x == 0) fail(a, kDevBadInput);
-            break;
-        }
-        for (int t = threadIdx.x; t < no; t += blockDim.x) {
-            s.a_row[nf + t] = a.lrow[o0 + t];
-            s.a_val[nf + t] = a.lval[o0 + t];
-        }
-        __syncthreads();
-        // ---- sort by (row, value bits); merge duplicate rows in that order
-        tail_radix_sort<false, false>(s.a_row, s.a_val, nullptr, s.t_row, s.t_val, nullptr, total, 0, 12, hist, tot);
-        const int tile = ((total + kTailWarps - 1) / kTailWarps + 31) & ~31;
-        const int t0 = min(total, w * tile), t1 = min(total, t0 + tile);
-        int heads = 0;
-        for (int base = t0; base < t1; base += kWarp) {
-            const int i = base + lane;
-            const bool head = i < t1 && (i == 0 || s.a_row[i - 1] != s.a_row[i]);
-            heads += __popc(__ballot_sync(kFull, head));
-        }
-        int m0 = tail_tile_offset(heads, scan);
-        const int m = scan[kTailWarps];
-        for (int base = t0; base < t1; base += kWarp) {
-            const int i = base + lane;
-            const bool valid = i < t1;
-            const int32_t ri = valid ? s.a_row[i] : INT_MAX;
-            const bool head = valid && (i == 0 || s.a_row[i - 1] != ri);
-            const unsigned bal = __ballot_sync(kFull, head);
-            if (head) {
-                const int rank = m0 + __popc(bal & lt);
-                double acc = s.a_val[i];
-                int cnt = 1;
-                for (int j = i + 1; j < total && s.a_row[j] == ri; ++j) {
-                    acc = __dadd_rn(acc, s.a_val[j]);
-                    ++cnt;
+            __syncthreads();
+            // ---- sort by (row, value bits); merge duplicate rows in that order
+            cta_radix_sort<NT, false, false>(s.a_row, s.a_val, nullptr, s.t_row, s.t_val, nullptr, total, 0, 12, hist,
+                                             tot);
+            const int tile = ((total + NW - 1) / NW + 31) & ~31;
+            const int t0 = min(total, w * tile), t1 = min(total, t0 + tile);
+            int heads = 0;
+            for (int base = t0; base < t1; base += kWarp) {
+                const int i = base + lane;
+                const bool hd = i < t1 && (i == 0 || s.a_row[i - 1] != s.a_row[i]);
+                heads += __popc(__ballot_sync(kFull, hd));
+            }
+            if (lane == 0) scan[w] = heads;
+            __syncthreads();
+            int m0 = 0;
+            for (int q = 0; q < NW; ++q) {
+                if (q < w) m0 += scan[q];
+                m += scan[q];
+            }
+            for (int base = t0; base < t1; base += kWarp) {
+                const int i = base + lane;
+                const bool valid = i < t1;
+                const int32_t ri = valid ? s.a_row[i] : INT_MAX;
+                const bool hd = valid && (i == 0 || s.a_row[i - 1] != ri);
+                const unsigned bal = __ballot_sync(kFull, hd);
+                if (hd) {
+                    const int rank = m0 + __popc(bal & lt);
+                    double acc = s.a_val[i];
+                    int cnt = 1;
+                    for (int j = i + 1; j < total && s.a_row[j] == ri; ++j) {
+                        acc = __dadd_rn(acc, s.a_val[j]);
+                        ++cnt;
+                    }
+                    s.b_val[rank] = acc;
+                    s.b_row[rank] = ri;
+                    s.b_aux[rank] = ((long long)cnt << 32) | (long long)rank;
                 }
-                s.b_val[rank] = acc;
-                s.b_row[rank] = ri;
-                s.b_aux[rank] = ((long long)cnt << 32) | (long long)rank;
+                m0 += __popc(bal);
             }
-            m0 += __popc(bal);
-        }
-        __syncthreads();
-        // ---- sort by value (input in row order: the value bytes suffice)
-        tail_radix_sort<true, true>(s.b_row, s.b_val, s.b_aux, s.t_row, s.t_val, s.t_aux, m, 4, 12, hist, tot);
-        // ---- prefix sums: 32-wide Kogge-Stone chunks (warp c % 32 takes
-        // chunk c), the chunk totals in t_val; then the carries chained in
-        // chunk order by one thread, as the warp path carries them
-        const int nchunk = (m + kWarp - 1) / kWarp;
-        for (int c = w; c < nchunk; c += kTailWarps) {
-            const int i = c * kWarp + lane;
-            double v = i < m ? s.b_val[i] : 0.0;
+            __syncthreads();
+            // ---- sort by value (input in row order: the value bytes suffice)
+            cta_radix_sort<NT, true, true>(s.b_row, s.b_val, s.b_aux, s.t_row, s.t_val, s.t_aux, m, 4, 12, hist, tot);
+            // ---- prefix sums as above, the chunk totals in t_val
+            const int nchunk = (m + kWarp - 1) / kWarp;
+            for (int c = w; c < nchunk; c += NW) {
+                const int i = c * kWarp + lane;
+                double v = i < m ? s.b_val[i] : 0.0;
 #pragma unroll
-            for (int off = 1; off < kWarp; off <<= 1) {
-                const double t = __shfl_up_sync(kFull, v, off);
-                if (lane >= off) v = __dadd_rn(v, t);
-            }
-            if (i < m) s.a_val[i] = v;
-            if (lane == kWarp - 1) s.t_val[c] = v;
-        }
-        __syncthreads();
-        if (w == 0) {
-            // t_val[c] becomes the carry into chunk c (c >= 1): one lane adds
-            // the totals in chunk order, 32 at a time read into registers
-            double carry = 0.0;
-            for (int c0 = 0; c0 < nchunk; c0 += kWarp) {
-                const double tl = c0 + lane < nchunk ? s.t_val[c0 + lane] : 0.0;
-                double cin = 0.0;
-                for (int q = 0; q < kWarp && c0 + q < nchunk; ++q) {
-                    const double tq = __shfl_sync(kFull, tl, q);
-                    if (lane == q) cin = carry;  // carry into chunk c0 + q
-                    carry = (c0 + q == 0) ? tq : __dadd_rn(carry, tq);
+                for (int off = 1; off < kWarp; off <<= 1) {
+                    const double t = __shfl_up_sync(kFull, v, off);
+                    if (lane >= off) v = __dadd_rn(v, t);
                 }
-                if (c0 + lane < nchunk) s.t_val[c0 + lane] = cin;
+                if (i < m) s.a_val[i] = v;
+                if (lane == kWarp - 1) s.t_val[c] = v;
             }
-        }
-        __syncthreads();
-        for (int i = kWarp + threadIdx.x; i < m; i += blockDim.x) s.a_val[i] = __dadd_rn(s.t_val[i / kWarp], s.a_val[i]);
-        __syncthreads();
-        const double S = s.a_val[m - 1];
-        // ---- L column k into the pool (row order), D_k
-        if (threadIdx.x == 0) {
-            const unsigned long long got = atomicAdd(a.pool_cursor, (unsigned long long)m);
-            sh_base = (long long)got;
-            if ((int64_t)got + m > a.pool_cap) {
-                fail(a, kDevCapacity);
-                sh_stop = 1;
-            } else {
+            __syncthreads();
+            if (w == 0) {
+                double carry = 0.0;
+                for (int c0 = 0; c0 < nchunk; c0 += kWarp) {
+                    const double tl = c0 + lane < nchunk ? s.t_val[c0 + lane] : 0.0;
+                    double cin = 0.0;
+                    for (int q = 0; q < kWarp && c0 + q < nchunk; ++q) {
+                        const double tq = __shfl_sync(kFull, tl, q);
+                        if (lane == q) cin = carry;  // carry into chunk c0 + q
+                        carry = (c0 + q == 0) ? tq : __dadd_rn(carry, tq);
+                    }
+                    if (c0 + lane < nchunk) s.t_val[c0 + lane] = cin;
+                }
+            }
+            __syncthreads();
+            for (int i = kWarp + tid; i < m; i += NT) s.a_val[i] = __dadd_rn(s.t_val[i / kWarp], s.a_val[i]);
+            if (tid == 0) sh_base = (int64_t)atomicAdd(a.pool_cursor, (unsigned long long)m);
+            __syncthreads();
+            const double S = s.a_val[m - 1];
+            const int64_t pbase = sh_base;
+            if (pbase + m > a.pool_cap) {
+                if (tid == 0) fail(a, kDevCapacity);
+                break;
+            }
+            if (tid == 0) {
                 a.diag[k] = S;
-                a.pstart[k] = (int64_t)got;
+                a.pstart[k] = pbase;
                 a.pcnt[k] = m;
             }
-        }
-        __syncthreads();
-        if (sh_stop) break;
-        const int64_t pbase = sh_base;
-        fills += m - 1;
-        for (int i = threadIdx.x; i < m; i += blockDim.x) {
-            const int p = (int)(s.b_aux[i] & 0xffffffffll);
-            a.prow[pbase + p] = s.b_row[i];
-            a.pval[pbase + p] = __ddiv_rn(s.b_val[i], S);
-        }
-        // ---- clique sampling (the same search predicate as the warp path),
-        // searching a shared-memory copy of the prefix sums when it fits
-        const double* C = s.a_val;
-        if (m <= a.tail_cdf_cap) {
-            double* cs = reinterpret_cast<double*>(smem + sizeof(int) * kTailIntWords);
-            for (int i = threadIdx.x; i < m; i += blockDim.x) cs[i] = s.a_val[i];
-            __syncthreads();
-            C = cs;
-        }
-        bool ok = true;
-        for (int i = threadIdx.x; i < m - 1; i += blockDim.x) {
-            const double ci = C[i];
-            const double rem_i = __dsub_rn(S, ci);
-            const double target = __dmul_rn(sample_uniform(a.seed, k, i), rem_i);
-            int lo = i + 1, hi = m;
-            while (lo < hi) {
-                const int mid = lo + ((hi - lo) >> 1);
-                if (__dsub_rn(C[mid], ci) < target) lo = mid + 1;
-                else hi = mid;
+            for (int i = tid; i < m; i += NT) {
+                const int p = (int)(s.b_aux[i] & 0xffffffffll);
+                a.prow[pbase + p] = s.b_row[i];
+                a.pval[pbase + p] = __ddiv_rn(s.b_val[i], S);
+                atomicMax(a.level + s.b_row[i], lk);
             }
-            const int j = lo < m ? lo : m - 1;
-            const int32_t r_i = s.b_row[i], r_j = s.b_row[j];
-            const int32_t grow = r_i > r_j ? r_i : r_j;
-            const int32_t gcol = r_i > r_j ? r_j : r_i;
-            const double gval = __ddiv_rn(__dmul_rn(s.b_val[i], rem_i), S);
-            if (!append_fill(a, gcol, grow, gval)) ok = false;
-            atomicAdd(a.dep + grow, 1);
+            // clique sampling over a shared-memory copy of the prefix sums when it fits
+            const double* C = s.a_val;
+            if (m <= Plan::kCdf) {
+                double* cs = reinterpret_cast<double*>(smem + 4 * Plan::kRadixWords);
+                for (int i = tid; i < m; i += NT) cs[i] = s.a_val[i];
+                __syncthreads();
+                C = cs;
+            }
+            for (int i = tid; i < m - 1; i += NT) {
+                const double rem_i = __dsub_rn(S, C[i]);
+                const int32_t ri = s.b_row[i], rj = s.b_row[sample_partner(a, k, i, m, C, rem_i)];
+                const int32_t grow = ri > rj ? ri : rj;
+                if (!append_fill(a, ri > rj ? rj : ri, grow, __ddiv_rn(__dmul_rn(s.b_val[i], rem_i), S))) ok = false;
+                atomicAdd(a.dep + grow, 1);
+            }
+            __threadfence();
+            if (__syncthreads_or(!ok)) {
+                if (tid == 0) fail(a, kDevCapacity);
+                break;
+            }
+            for (int i = tid; i < m; i += NT) release_row(a, s.b_row[i], (int)(s.b_aux[i] >> 32));
+            fills += m - 1;
+            if (lock >= 0) {
+                __syncthreads();
+                if (w == 0) release_huge(a, lane, lock);
+            }
         }
-        // rows of L column k are one level below k (the solve schedules)
-        const int lk = ld_relaxed(a.level + k) + 1;
-        for (int i = threadIdx.x; i < m; i += blockDim.x) atomicMax(a.level + s.b_row[i], lk);
-        if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0) fail(a, kDevCapacity);
-            break;
-        }
-        // fills, pool writes and levels visible before any neighbour is
-        // released: each neighbour's counter drops by its multiplicity
-        __threadfence();
-        __syncthreads();
-        for (int i = threadIdx.x; i < m; i += blockDim.x)
-            atom_add_acq_rel(a.dep + s.b_row[i], -(int)(s.b_aux[i] >> 32));
-        if (threadIdx.x == 0) atomicAdd(a.counters + kDone, 1);
+        if (tid == 0) atomicAdd(a.counters + kDone, 1);
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        atomicMax(a.counters + kMaxGather, max_gather);
-        atomicAdd(a.pool_cursor + 1, (unsigned long long)fills);
+    if (tid == 0) {
+        if (max_gather) atomicMax(a.counters + kMaxGather, max_gather);
+        if (fills) atomicAdd(a.pool_cursor + 1, (unsigned long long)fills);
     }
 }
 
-size_t tail_smem_bytes() { return sizeof(int) * (size_t)kTailIntWords + sizeof(double) * (size_t)kTailCdfCap; }
+using CtaMid = CtaPlan<256, 4>;
+using CtaTail = CtaPlan<1024, 4>;
 
 // ---- setup kernels --------------------------------------------------------
 
@@ -1636,6 +2029,15 @@ int factor_resident_grid(int block, int smem_slab, int device) {
     return per_sm * sms;
 }
 
+int factor_cta_grid(int device) {
+    const void* fn = (const void*)factor_cta_kernel<256, 4>;
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CtaMid::kBytes);
+    int per_sm = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, CtaMid::kBytes) != cudaSuccess) return 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return per_sm * sms;
+}
+
 cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s) {
     FactorArgs a;
     a.n = w.n;
@@ -1672,20 +2074,31 @@ cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s
     a.smem_slab = cfg.smem_slab;
     a.smem_region = smem_region_bytes(cfg.smem_slab);
     a.timeout_ns = (unsigned long long)(cfg.timeout_s * 1e9);
-    a.tail = cfg.tail > 0 && cfg.tail < w.n ? w.n - cfg.tail : w.n;
-    a.tail_cdf_cap = kTailCdfCap;
+    // [0, mid) a warp per vertex, [mid, tail) a 256-thread CTA, [tail, n) a
+    // 1024-thread CTA (a tail of every vertex keeps the warp path for none)
+    const int32_t tail = cfg.tail > 0 && cfg.tail < w.n ? w.n - cfg.tail : w.n;
+    const int32_t mid = std::min<int32_t>(tail, w.n - std::min<int32_t>(w.n, cfg.cta));
+    a.tail = mid;
     a.gsize = cfg.gsize;
     size_t smem = factor_smem_bytes(cfg.block, cfg.smem_slab);
     cudaError_t e = cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    factor_kernel<<<cfg.grid, cfg.block, smem, s>>>(a);
-    RCHOL_TRY(cudaGetLastError());
-    if (a.tail < w.n) {
-        // the tail after the rest is eliminated: one CTA per shared slab,
-        // each a vertex at a time, claimed in index order
-        const size_t tsmem = tail_smem_bytes();
-        RCHOL_TRY(cudaFuncSetAttribute(factor_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
-        factor_tail_kernel<<<w.nhuge, kTailThreads, tsmem, s>>>(a);
+    if (mid > 0) {
+        factor_kernel<<<cfg.grid, cfg.block, smem, s>>>(a);
+        RCHOL_TRY(cudaGetLastError());
+    }
+    if (mid < tail) {
+        const void* fn = (const void*)factor_cta_kernel<256, 4>;
+        RCHOL_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CtaMid::kBytes));
+        factor_cta_kernel<256, 4><<<std::min<int32_t>(cfg.cta_grid, tail - mid), 256, CtaMid::kBytes, s>>>(
+            a, mid, tail, kMidTicket);
+        RCHOL_TRY(cudaGetLastError());
+    }
+    if (tail < w.n) {
+        const void* fn = (const void*)factor_cta_kernel<1024, 4>;
+        RCHOL_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CtaTail::kBytes));
+        factor_cta_kernel<1024, 4><<<std::min<int32_t>(current_sm_count(), w.n - tail), 1024, CtaTail::kBytes, s>>>(
+            a, tail, w.n, kTailTicket);
         RCHOL_TRY(cudaGetLastError());
     }
     return cudaSuccess;

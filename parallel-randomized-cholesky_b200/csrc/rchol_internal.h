@@ -321,7 +321,9 @@ struct FactorLaunch {
     int smem_slab = 256;      // entries per warp slab in shared memory
     uint64_t seed = 1;
     double timeout_s = 20.0;
-    int32_t tail = 0;         // the last `tail` vertices are eliminated by one cooperative CTA (0: none)
+    int32_t tail = 0;         // the last `tail` vertices are eliminated by a 1024-thread CTA each (0: none)
+    int32_t cta = 0;          // the last `cta` vertices (before the tail) by a 256-thread CTA each
+    int cta_grid = 1;         // CTAs of that pass
     int32_t* gsize = nullptr; // device [n]: gathered entries of each vertex (null: not recorded)
 };
 
@@ -331,6 +333,8 @@ cudaError_t launch_count_lower(const DevCsc& A, int32_t* lower_cnt, int32_t* hug
 cudaError_t launch_init_factor_state(FactorWork& w, cudaStream_t s);
 cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s);
 int factor_resident_grid(int block, int smem_slab, int device);
+// Resident CTAs of the 256-thread cooperative pass.
+int factor_cta_grid(int device);
 size_t factor_smem_bytes(int block, int smem_slab);
 
 // Assemble Lc/Lr (and FP32 copies) from the pool; drop the last vertex when

@@ -303,6 +303,31 @@ def test_cooperative_tail_is_bit_exact(case, tail):
         ctx.close()
 
 
+@pytest.mark.parametrize("N,tail", [(31, False), (32, False), (33, False), (64, False), (65, False), (256, False),
+                                    (257, False), (512, False), (513, False), (1024, False), (1025, False),
+                                    (1024, True), (1025, True), (2049, True), (4096, True), (4097, True)])
+def test_cta_elimination_list_sizes(N, tail):
+    """A late vertex that gathers N entries, around the list sizes at which
+    the cooperative kernels change their code (one warp, 1, 2 and 4 entries
+    per thread, slabs in global memory), with 256 threads (the last eighth of
+    the vertices) and with 1024 (tail_vertices): bit-exact."""
+    rng = np.random.default_rng(N)
+    early = 8 if tail else 8 * (N + 40)
+    n = early + 1 + N
+    hub = early
+    a = np.concatenate([np.arange(early), np.full(N, hub), np.arange(hub + 1, n - 1)])
+    b = np.concatenate([np.arange(1, early + 1), np.arange(hub + 1, n), np.arange(hub + 2, n)])
+    # repeated weights: ties in the value sort break on the row
+    w = rng.integers(1, 5, len(a)) * np.exp(rng.integers(0, 2, len(a)) * rng.uniform(-3, 3, len(a)))
+    d = np.bincount(a, weights=w, minlength=n) + np.bincount(b, weights=w, minlength=n)
+    i = np.arange(n)
+    r, c, v = np.concatenate([a, b, i]), np.concatenate([b, a, i]), np.concatenate([-w, -w, d])
+    orc = OracleProblem(n, r, c, v).factor(seed=3)
+    gpu, info = _gpu_factor(n, r, c, v, False, 3, **(dict(tail_vertices=N + 1) if tail else {}))
+    _compare(gpu, orc)
+    assert info.max_gather >= N
+
+
 def test_autotune_choices_are_used_and_cached():
     """rchol_autotune profiles the gathers, keeps only choices that time
     faster, writes them into the context's options (the next factorization
