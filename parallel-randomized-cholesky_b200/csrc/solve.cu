@@ -197,27 +197,52 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
     return false;
 }
 
-// Column sums of the blocks' partials by the whole last block: thread t adds
-// every (kBlock / K)-th partial of column t % K, then a fixed tree joins the
-// threads of a column (deterministic).  One thread per column adding all the
-// partials (1184 for the SpMV's grid) was a chain of L2 round trips: it took
-// 16 of the 23 us of a 2867-unknown SpMV launch.
+// Column sums of the blocks' partials in block order.  The last block brings
+// the partials to shared memory together, a tile at a time and two ahead, and
+// thread c adds column c: with the loads in the adding thread's own chain the
+// 1184 partials of a SpMV launch took 10 of its 23 us on 2867 unknowns.  (A tree
+// would be faster still, but any other grouping moves the iterates of loosely
+// converged solves by up to their error.)  The tile is small because a kernel's
+// shared memory comes out of the L1 that its gathers live in: with 8 KB instead
+// of 4 the k = 8 SpMV took 72 us, not 60; 32 columns need the larger tile (258
+// against 283 us).
+template <int K>
+constexpr int sum_tile() {
+    return K >= 16 ? 1024 : 512;
+}
+
 template <int K>
 __device__ void sum_partials(const double* part, int nblocks, double* out) {
-    __shared__ double red[kBlock];
-    constexpr int G = kBlock / K;
-    const int c = threadIdx.x % K, g = threadIdx.x / K;
-    double s = 0.0;
-#pragma unroll 4
-    for (int b = g; b < nblocks; b += G) s += __ldcg(part + (size_t)b * K + c);
-    red[threadIdx.x] = s;
-    __syncthreads();
+    constexpr int kSumTile = sum_tile<K>();
+    __shared__ double tile[kSumTile];
+    constexpr int B = kSumTile / K;     // blocks per tile
+    constexpr int U = kSumTile / kBlock;
+    const int total = nblocks * K;
+    double s = 0.0, next[2][U];         // the next two tiles, on their way
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-        if (g < o) red[threadIdx.x] += red[threadIdx.x + o * K];
+    for (int d = 0; d < 2; ++d)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = d * kSumTile + u * kBlock + threadIdx.x;
+            next[d][u] = q < total ? __ldcg(part + q) : 0.0;
+        }
+    for (int b0 = 0; b0 < nblocks; b0 += B) {
+        const int nb = min(B, nblocks - b0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = (b0 + 2 * B) * K + u * kBlock + threadIdx.x;
+            tile[u * kBlock + threadIdx.x] = next[0][u];
+            next[0][u] = next[1][u];
+            next[1][u] = q < total ? __ldcg(part + q) : 0.0;
+        }
+        __syncthreads();
+        if (threadIdx.x < K) {
+#pragma unroll 8
+            for (int b = 0; b < nb; ++b) s += tile[b * K + threadIdx.x];
+        }
         __syncthreads();
     }
-    if (threadIdx.x < K) out[threadIdx.x] = red[threadIdx.x];
+    if (threadIdx.x < K) out[threadIdx.x] = s;
     __syncthreads();
 }
 
@@ -491,7 +516,7 @@ __global__ void __launch_bounds__(kBlock, 8) spmv_update_kernel(SolveArgs a) {
     if (last_block(&a.sc->ticket[1])) {
         sum_partials<K>(a.part, gridDim.x, a.sc->pq);
         if (a.n_lrows > 0) {
-            // the long rows' terms, summed the same way
+            // the long rows' terms, in row order
             double* t = a.lr_dot + (size_t)a.n_lrows * K;
             sum_partials<K>(a.lr_dot, a.n_lrows, t);
             if (threadIdx.x < K) a.sc->pq[threadIdx.x] += t[threadIdx.x];
@@ -520,11 +545,14 @@ constexpr int kSpmvChunk = RCHOL_SPMV_CHUNK;  // entries staged per warp and chu
 // entry order, then the threads' sums in a fixed tree; the same q, p, y and
 // p.q term as the tile and sliced-ELL kernels, which skip these rows.
 
-// pq += the long rows' p.q terms (spmv_long_kernel ran first), in a fixed
-// tree.  Called by every thread of the SpMV's last block.
+// pq += the long rows' p.q terms (spmv_long_kernel ran first): each thread
+// every kBlock-th term in order, then the threads in a fixed tree.  Called
+// by every thread of the SpMV's last block.
 __device__ void add_long_row_terms(SolveArgs& a) {
     if (a.n_lrows == 0) return;
-    sum_partials<1>(a.lr_dot, a.n_lrows, a.lr_dot + a.n_lrows);
+    double lt[1] = {0.0};
+    for (int k = threadIdx.x; k < a.n_lrows; k += blockDim.x) lt[0] += a.lr_dot[k];
+    block_partials<1>(lt, a.lr_dot + a.n_lrows);
     if (threadIdx.x == 0) a.sc->pq[0] += a.lr_dot[a.n_lrows];
 }
 
@@ -1969,7 +1997,7 @@ cudaError_t pcg_profile(PcgSolver* s, const double* dB, double* dX, int reps, fl
 // right-hand side).  Rows are grouped by system; the dot products reduce
 // over fixed row chunks (a chunk spans at most two systems) and then over
 // the chunks of each system in order, so the sums are deterministic.
-// One iteration: batch_spmv (q, p, p.q -> alpha per pair), fwd (x, r, y),
+// One iteration: batch_spmv (q, p), batch_pq (p.q -> alpha per pair), fwd (x, r, y),
 // bwd (z), batch_dots (r.r, r.z -> convergence, beta per pair).
 // ===========================================================================
 
@@ -2023,41 +2051,66 @@ __device__ void chunk_store(double va, double vb, double* out /* [2][K] */) {
     __syncthreads();
 }
 
-// Sum of the chunk partials of every (system, column) pair into out[pair]: a
-// warp per system, column lane % K, 32 / K chunks per load, fixed tree.
+// Sum of the chunk partials of every (system, column) pair into out[pair]:
+// lanes over the system's chunks, fixed tree.  A warp takes 4 pairs at a time,
+// so that their loads and trees overlap.
 template <int K>
 __device__ void reduce_pairs(const BatchArgs& a, const double* part, double* out) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    constexpr int S = 32 / K;
-    const int c = lane % K, g = lane / K;
-    for (int sys = w; sys < a.nsys; sys += kBlock / 32) {
-        const int64_t r0 = a.sys_off[sys], r1 = a.sys_off[sys + 1];
-        double t = 0.0;
-        if (r1 > r0) {
-            const int64_t c0 = r0 / a.chunk, c1 = (r1 - 1) / a.chunk;
-            // a chunk that starts before the system holds it in its second slot
-#pragma unroll 8
-            for (int64_t ch = c0 + g; ch <= c1; ch += S)
-                t += __ldcg(part + (size_t)ch * 2 * K + (ch * a.chunk < r0 ? K : 0) + c);
+    const int pairs = a.nsys * K;
+    for (int p0 = w * 4; p0 < pairs; p0 += (kBlock / 32) * 4) {
+        double t[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int pr = min(p0 + q, pairs - 1);
+            const int sys = pr / K, c = pr % K;
+            const int64_t r0 = a.sys_off[sys], r1 = a.sys_off[sys + 1];
+            t[q] = 0.0;
+            if (r1 > r0) {
+                const int64_t c0 = r0 / a.chunk, c1 = (r1 - 1) / a.chunk;
+                // a chunk that starts before the system holds it in its second slot
+                for (int64_t ch = c0 + lane; ch <= c1; ch += 32)
+                    t[q] += __ldcg(part + (size_t)ch * 2 * K + (ch * a.chunk < r0 ? K : 0) + c);
+            }
         }
 #pragma unroll
-        for (int o = 16; o >= K; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
-        if (lane < K) out[sys * K + lane] = t;
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) t[q] += __shfl_xor_sync(kFull, t[q], o);
+        if (lane < 4 && p0 + lane < pairs) out[p0 + lane] = lane == 0 ? t[0] : lane == 1 ? t[1] : lane == 2 ? t[2] : t[3];
     }
     __syncthreads();
 }
 
-// Row loop of one chunk: fn(row, column) returns the row's contribution.
+// Row loop of one chunk: the sum of the products fn(row, column) = {x, y} over the
+// thread's rows, fused multiply-adds in row order, apart for the chunk's first system (va) and its second (vb).  The
+// chunks are few and long (they fix the sums' grouping), so a thread fetches
+// kChunkRows rows before it adds them: a row at a time, the dots' loop was 128
+// round trips and most of their time.
+constexpr int kChunkRows = 8;
+
 template <int K, typename F>
-__device__ void chunk_rows(const BatchArgs& a, int64_t ch, F fn, double& va, double& vb) {
+__device__ __forceinline__ void chunk_rows(const BatchArgs& a, int64_t ch, F fn, double& va, double& vb) {
     const int64_t r0 = ch * a.chunk;
     const int64_t r1 = min((int64_t)a.n, r0 + a.chunk);
-    const int first = a.seg[r0];
+    const int64_t second = a.sys_off[a.seg[r0] + 1];  // first row of the next system
     const int c = threadIdx.x % K;
-    for (int64_t i = r0 + threadIdx.x / K; i < r1; i += kBlock / K) {
-        const double v = fn(i, c);
-        if (a.seg[i] == first) va += v;
-        else vb += v;
+    constexpr int step = kBlock / K;
+    int64_t i = r0 + threadIdx.x / K;
+    for (; i + (kChunkRows - 1) * step < r1; i += kChunkRows * step) {
+        double2 v[kChunkRows];
+#pragma unroll
+        for (int u = 0; u < kChunkRows; ++u) v[u] = fn(i + u * step, c);
+#pragma unroll
+        for (int u = 0; u < kChunkRows; ++u) {
+            if (i + u * step < second) va = __fma_rn(v[u].x, v[u].y, va);
+            else vb = __fma_rn(v[u].x, v[u].y, vb);
+        }
+    }
+    for (; i < r1; i += step) {
+        const double2 v = fn(i, c);
+        if (i < second) va = __fma_rn(v.x, v.y, va);
+        else vb = __fma_rn(v.x, v.y, vb);
     }
 }
 
@@ -2073,7 +2126,7 @@ __global__ void __launch_bounds__(kBlock) batch_init_kernel(BatchArgs a) {
             a.p[o] = 0.0;
             a.q[o] = 0.0;
             a.y[o] = pending_value();
-            return bv * bv;
+            return make_double2(bv, bv);
         }, va, vb);
         chunk_store<K>(va, vb, a.part + (size_t)ch * 2 * K);
     }
@@ -2099,21 +2152,33 @@ __global__ void __launch_bounds__(kBlock) batch_init_kernel(BatchArgs a) {
     }
 }
 
+// q = A z + beta q, p = z + beta p, y reset: K lanes per row over the whole
+// grid.  The p.q sums, which keep the chunks' grouping, are batch_pq_kernel's: in
+// one kernel over the chunks (72 of them for 293 k rows) half of the SMs idled.
 template <int K>
 __global__ void __launch_bounds__(kBlock) batch_spmv_kernel(BatchArgs a) {
+    if (ld_relaxed(&a.sc->done)) return;
+    const int c = threadIdx.x % K;
+    const int64_t ngroups = (int64_t)gridDim.x * blockDim.x / K;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / K; i < a.n; i += ngroups) {
+        const double beta = a.s.beta[(size_t)a.seg[i] * K + c];
+        const double sum = row_dot_plain<K>(a.a_idx, a.a_val, a.a_ptr[i], a.a_ptr[i + 1], a.z, c);
+        const size_t o = (size_t)i * K + c;
+        a.q[o] = sum + beta * a.q[o];
+        a.p[o] = a.z[o] + beta * a.p[o];
+        a.y[o] = pending_value();
+    }
+}
+
+// p.q -> alpha per pair
+template <int K>
+__global__ void __launch_bounds__(kBlock) batch_pq_kernel(BatchArgs a) {
     if (ld_relaxed(&a.sc->done)) return;
     for (int64_t ch = blockIdx.x; ch < a.nchunks; ch += gridDim.x) {
         double va = 0.0, vb = 0.0;
         chunk_rows<K>(a, ch, [&](int64_t i, int c) {
-            const double beta = a.s.beta[(size_t)a.seg[i] * K + c];
-            const double sum = row_dot_plain<K>(a.a_idx, a.a_val, a.a_ptr[i], a.a_ptr[i + 1], a.z, c);
             const size_t o = (size_t)i * K + c;
-            const double qi = sum + beta * a.q[o];
-            const double pi = a.z[o] + beta * a.p[o];
-            a.q[o] = qi;
-            a.p[o] = pi;
-            a.y[o] = pending_value();
-            return pi * qi;
+            return make_double2(a.p[o], a.q[o]);
         }, va, vb);
         chunk_store<K>(va, vb, a.part + (size_t)ch * 2 * K);
     }
@@ -2134,25 +2199,16 @@ __global__ void __launch_bounds__(kBlock) batch_dots_kernel(BatchArgs a) {
     if (ld_relaxed(&a.sc->done)) return;
     double* part_rr = a.part;
     double* part_rz = a.part + (size_t)a.nchunks * 2 * K;
-    for (int64_t ch = blockIdx.x; ch < a.nchunks; ch += gridDim.x) {
-        double va = 0.0, vb = 0.0, wa = 0.0, wb = 0.0;
-        const int64_t r0 = ch * a.chunk;
-        const int64_t r1 = min((int64_t)a.n, r0 + a.chunk);
-        const int first = a.seg[r0];
-        const int c = threadIdx.x % K;
-        for (int64_t i = r0 + threadIdx.x / K; i < r1; i += kBlock / K) {
+    // a chunk's two dots by two CTAs
+    for (int64_t u = blockIdx.x; u < 2 * (int64_t)a.nchunks; u += gridDim.x) {
+        const int64_t ch = u >> 1;
+        const double* other = (u & 1) ? a.z : a.r;
+        double va = 0.0, vb = 0.0;
+        chunk_rows<K>(a, ch, [&](int64_t i, int c) {
             const size_t o = (size_t)i * K + c;
-            const double ri = a.r[o], zi = a.z[o];
-            if (a.seg[i] == first) {
-                va += ri * ri;
-                wa += ri * zi;
-            } else {
-                vb += ri * ri;
-                wb += ri * zi;
-            }
-        }
-        chunk_store<K>(va, vb, part_rr + (size_t)ch * 2 * K);
-        chunk_store<K>(wa, wb, part_rz + (size_t)ch * 2 * K);
+            return make_double2(a.r[o], other[o]);
+        }, va, vb);
+        chunk_store<K>(va, vb, ((u & 1) ? part_rz : part_rr) + (size_t)ch * 2 * K);
     }
     if (last_block(&a.sc->ticket[3])) {
         reduce_pairs<K>(a, part_rr, a.s.rr);
@@ -2201,7 +2257,7 @@ __global__ void __launch_bounds__(kBlock) batch_true_kernel(BatchArgs a) {
         chunk_rows<K>(a, ch, [&](int64_t i, int c) {
             const double sum = row_dot_plain<K>(a.a_idx, a.a_val, a.a_ptr[i], a.a_ptr[i + 1], a.x, c);
             const double t = a.b[(size_t)i * K + c] - sum;
-            return t * t;
+            return make_double2(t, t);
         }, va, vb);
         chunk_store<K>(va, vb, a.part + (size_t)ch * 2 * K);
     }
@@ -2220,8 +2276,9 @@ class BatchSolver {
     double* pool = nullptr;          // per-pair scalars
     int* ipool = nullptr;
     double* part = nullptr;
-    int grid = 0;
-    void *k_init = nullptr, *k_spmv = nullptr, *k_dots = nullptr, *k_true = nullptr;
+    int grid = 0, grid2 = 0, grid_rows = 0;  // CTAs over the chunks (two dots), over the rows
+    void *k_init = nullptr, *k_spmv = nullptr, *k_pq = nullptr, *k_dots = nullptr, *k_true = nullptr;
+
     cudaGraphExec_t graph = nullptr;
     const double* gb = nullptr;
     double* gx = nullptr;
@@ -2259,10 +2316,11 @@ class BatchSolver {
         BatchArgs a = args(b, x);
         SolveArgs sa = solve_args(b, x);
         cudaError_t e;
-        if ((e = launch(k_spmv, grid, &a)) != cudaSuccess) return e;
+        if ((e = launch(k_spmv, grid_rows, &a)) != cudaSuccess) return e;
+        if ((e = launch(k_pq, grid, &a)) != cudaSuccess) return e;
         if ((e = launch(base->k_fwd, base->grid_fwd, &sa)) != cudaSuccess) return e;
         if ((e = launch(base->k_bwd, base->grid_bwd, &sa)) != cudaSuccess) return e;
-        return launch(k_dots, grid, &a);
+        return launch(k_dots, grid2, &a);
     }
 };
 
@@ -2270,6 +2328,7 @@ template <int K>
 static void bind_batch(BatchSolver* s) {
     s->k_init = (void*)batch_init_kernel<K>;
     s->k_spmv = (void*)batch_spmv_kernel<K>;
+    s->k_pq = (void*)batch_pq_kernel<K>;
     s->k_dots = (void*)batch_dots_kernel<K>;
     s->k_true = (void*)batch_true_kernel<K>;
 }
@@ -2297,15 +2356,8 @@ BatchSolver* batch_create(const DevCsc& A, const DevFactor& F, const SolveConfig
         case 32: bind_batch<32>(s); break;
         default: *err = cudaErrorInvalidValue; batch_destroy(s); return nullptr;
     }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    // enough chunks for 4 CTAs per SM, of at least 128 rows where the systems
-    // allow it (a 293 k-row batch of 12 systems: 72 chunks of 4096 rows left
-    // half of the SMs idle)
     int64_t chunk = 32;
-    while (chunk * 2 <= std::min<int64_t>(minsys, 4096) &&
-           (chunk < 128 || A.n / (chunk * 2) >= (int64_t)sms * 4))
-        chunk *= 2;
+    while (chunk * 2 <= std::min<int64_t>(minsys, 4096)) chunk *= 2;
     const int K = cfg.k;
     const int64_t pairs = (int64_t)nsys * K;
     BatchArgs& a = s->ba;
@@ -2356,6 +2408,10 @@ BatchSolver* batch_create(const DevCsc& A, const DevFactor& F, const SolveConfig
     a.s.rzn = P + 8 * pairs;
     a.s.active = s->ipool;
     a.s.iters = s->ipool + pairs;
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    s->grid_rows = (int)std::min<int64_t>(ceil_div((int64_t)A.n * K, kBlock), (int64_t)sms * 8);
+    s->grid2 = (int)std::min<int64_t>(2 * (int64_t)a.nchunks, (int64_t)sms * 8);
     s->grid = (int)std::min<int64_t>(a.nchunks, (int64_t)sms * 8);
     return s;
 }
@@ -2403,7 +2459,7 @@ cudaError_t batch_solve(BatchSolver* s, const double* dB, double* dX, BatchResul
         sa.update = 0;
         if ((e = s->launch(b->k_fwd, b->grid_fwd, &sa)) != cudaSuccess) return e;
         if ((e = s->launch(b->k_bwd, b->grid_bwd, &sa)) != cudaSuccess) return e;
-        if ((e = s->launch(s->k_dots, s->grid, &a)) != cudaSuccess) return e;
+        if ((e = s->launch(s->k_dots, s->grid2, &a)) != cudaSuccess) return e;
     }
     cudaEventRecord(b->ev1, b->stream);
     res->kernel_launches = 4;
@@ -2416,7 +2472,7 @@ cudaError_t batch_solve(BatchSolver* s, const double* dB, double* dX, BatchResul
             for (int u = 0; u < b->cfg.unroll; ++u)
                 if ((e = s->iteration(dB, dX)) != cudaSuccess) return e;
         }
-        res->kernel_launches += 4 * b->cfg.unroll;
+        res->kernel_launches += 5 * b->cfg.unroll;
         if ((e = cudaMemcpyAsync(b->sc_host, b->sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, b->stream)) !=
             cudaSuccess)
             return e;
