@@ -77,9 +77,9 @@ typedef struct rchol_opts {
                                  power-law graphs); 0 = none; rchol_autotune picks it */
     int rhs_block;            /* multi-RHS PCG: solve k right-hand sides in blocks of this width
                                  (1, 2, 4, 8, 16, 32; 0 = all k at once); rchol_autotune picks it */
-    int bwd_head;             /* one-RHS PCG (exact backward levels): solve the narrow first levels
-                                 of the backward DAG in one CTA with the values in shared memory
-                                 before the persistent kernel (default 1; 0 = off) */
+    int bwd_head;             /* one RHS (exact backward levels): solve the narrow last levels of the
+                                 forward DAG and first levels of the backward one in one cluster of
+                                 CTAs with the values in shared memory (default 1; 0 = off) */
 } rchol_opts;
 
 typedef struct rchol_factor_info {
@@ -109,7 +109,7 @@ typedef struct rchol_factor_info {
     const double* diag;       /* D [n] */
     int tail_vertices;        /* vertices eliminated by the cooperative tail pass */
     int solve_depth_b;        /* levels of the backward-solve DAG (exact levels) */
-    int bwd_head_levels;      /* backward levels solved by the one-CTA head kernel (0: none) */
+    int bwd_head_levels;      /* backward levels whose r.z terms form a sum of their own (0: none) */
     int bwd_head_rows;        /* rows in those levels */
 } rchol_factor_info;
 

@@ -564,20 +564,20 @@ cudaError_t dmalloc(T** p, int64_t n) {
     return cudaMalloc((void**)p, sizeof(T) * (size_t)(n > 0 ? n : 1));
 }
 
-// Level table of the backward schedule's first lvcap levels: lv[l] = {first
-// task, first slab unit, first position} of level l, written by the task that
-// opens the level (levels are contiguous in task order), plus the end of
-// the last level when it falls inside the table.  split_min receives the
-// lowest level holding a part task.
-__global__ void head_level_kernel(int32_t npt, const int4* __restrict__ pack, const int32_t* __restrict__ order,
-                                  const int32_t* __restrict__ level, int32_t n, int32_t lvcap, int4* lv,
-                                  int32_t* split_min) {
+// Level table of the levels l0 .. l0 + lvcap of one direction's schedule:
+// lv[l - l0] = {first task, first slab unit, first position} of level l,
+// written by the task that opens the level (levels are contiguous in task
+// order), plus the end of the last level when it falls inside the table.
+// split_min receives the lowest level below l0 + lvcap holding a part task.
+__global__ void level_table_kernel(int32_t npt, const int4* __restrict__ pack, const int32_t* __restrict__ order,
+                                   const int32_t* __restrict__ level, int32_t n, int32_t l0, int32_t lvcap, int4* lv,
+                                   int32_t* split_min) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < npt; t += stride) {
         const int4 d = pack[t];
-        const int32_t l = level[order[d.x]];
-        if (l > lvcap) continue;
-        if (t == 0 || level[order[pack[t - 1].x]] != l) lv[l] = make_int4((int)t, d.y, d.x, 0);
+        const int32_t l = level[order[d.x]] - l0;
+        if (l < 0 || l > lvcap) continue;
+        if (t == 0 || level[order[pack[t - 1].x]] - l0 != l) lv[l] = make_int4((int)t, d.y, d.x, 0);
         if (((d.z >> 11) & 1) && l < lvcap) atomicMin(split_min, l);
         if (t == npt - 1 && l + 1 <= lvcap) lv[l + 1] = make_int4(npt, d.y + (d.w & 0xff), n, 0);
     }
@@ -588,20 +588,16 @@ __global__ void invert_order_kernel(int32_t n, const int32_t* __restrict__ order
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride) pos[order[p]] = (int32_t)p;
 }
 
-// Head slab slots with row indices replaced by positions in order_b; a
-// position outside the head (which the level structure rules out) sets bad.
-__global__ void head_idx_kernel(int64_t nslots, const int32_t* __restrict__ pidx, const int32_t* __restrict__ pos,
-                                int32_t rows, int32_t* out, int32_t* bad) {
+// The slab slots of the positions p0 .. p0 + rows - 1 (see DevFactor::nf_idx).
+__global__ void narrow_idx_kernel(int64_t nslots, const int32_t* __restrict__ pidx, const int32_t* __restrict__ pos,
+                                  int32_t p0, int32_t rows, int32_t* out) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nslots; s += stride) {
         const int32_t j = pidx[s];
-        int32_t q = -1;
+        int32_t q = INT32_MIN;
         if (j >= 0) {
-            q = pos[j];
-            if (q >= rows) {
-                *bad = 1;
-                q = -1;
-            }
+            q = pos[j] - p0;
+            if (q < 0 || q >= rows) q = -1 - j;
         }
         out[s] = q;
     }
@@ -907,7 +903,7 @@ static cudaError_t build_pack(int32_t ntasks, const int2* tasks, const int32_t* 
 // from the rows of Lr (forward) and Lc (backward); FP32 values are copied
 // when the factor has them.
 static cudaError_t build_packs(DevFactor& f, const int32_t* level_f, const int32_t* level_b, int sign_b,
-                                 Scratch& sc, cudaStream_t s) {
+                                 int32_t** pos_out, Scratch& sc, cudaStream_t s) {
     const PackOut of{&f.pack_f, &f.cap_pdf, &f.pf_idx, &f.cap_pif, &f.pf_val, &f.cap_pvf, &f.pf_val32, &f.cap_pwf,
                      &f.slots_f, &f.npt_f, &f.nsplit_f, &f.split_f, &f.cap_sf, &f.psum_f, &f.cap_qf, &f.pcount_f,
                      &f.cap_cf, &f.srow_f, &f.cap_rf};
@@ -922,6 +918,7 @@ static cudaError_t build_packs(DevFactor& f, const int32_t* level_f, const int32
     int32_t* pos_f = nullptr;
     RCHOL_TRY(sc.get(&pos_f, std::max<int32_t>(f.n, 1)));
     (void)level_f;
+    *pos_out = pos_f;
     invert_order_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(f.n, f.order_f, pos_f);
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(build_pack(f.ntasks_f, f.tasks_f, f.order_f, f.lr_ptr, f.lr_idx, f.lr_val, f.lr_val32, pos_f, 1,
@@ -931,57 +928,83 @@ static cudaError_t build_packs(DevFactor& f, const int32_t* level_f, const int32
     return cudaSuccess;
 }
 
-// The backward head (see DevFactor::hb_nlev): levels from the first while
-// each holds at most kHeadMaxRows rows, kHeadMaxTasks tasks and no part
-// task, and the head's rows, level table and largest stage (FP64 values, so
-// that either value type fits) fit the kernel's shared memory.  Fewer than
-// kHeadMinLevels such levels leave the head empty.
-static cudaError_t build_bwd_head(DevFactor& f, const int32_t* levb, Scratch& sc, cudaStream_t s) {
-    f.hb_nlev = f.hb_ntask = f.hb_rows = f.hb_stage = 0;
-    const int32_t lvcap = std::min<int32_t>(f.depth_b, kHeadMaxLevels);
-    if (f.npt_b == 0 || lvcap < kHeadMinLevels) return cudaSuccess;
+static void clear_narrow(DevFactor& f) {
+    f.nf_task = f.nf_unit = f.nf_pos = f.nf_rows = f.nb_task = f.nb_rows = 0;
+    f.narrow_long = false;
+    f.hb_nlev = f.hb_ntask = f.hb_rows = 0;
+}
+
+// The narrow levels of both directions (see DevFactor::nf_rows) and the
+// levels whose r.z terms are summed apart (hb_nlev).
+static cudaError_t build_narrow(DevFactor& f, const int32_t* levf, const int32_t* levb, const int32_t* pos_f,
+                                Scratch& sc, cudaStream_t s) {
+    clear_narrow(f);
+    const int32_t cf = std::min<int32_t>(f.depth, kNarrowMaxLevels), lf0 = f.depth - cf;
+    const int32_t cb = std::min<int32_t>(f.depth_b, kNarrowMaxLevels);
+    if (f.npt_b == 0 || std::max(cf, cb) < kNarrowMinLevels) return cudaSuccess;
+    // both level tables behind two flag words, brought over in one copy
     int4* lv = nullptr;
-    int32_t* flags = nullptr;  // [0] lowest split level, [1] bad index
-    RCHOL_TRY(sc.get(&lv, (int64_t)lvcap + 1));
-    RCHOL_TRY(sc.get(&flags, 2));
-    const int32_t init[2] = {INT32_MAX, 0};
-    RCHOL_TRY(cudaMemcpyAsync(flags, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    head_level_kernel<<<grid_for(f.npt_b, 256), 256, 0, s>>>(f.npt_b, f.pack_b, f.order_b, levb, f.n, lvcap, lv,
-                                                             flags);
+    const int64_t nlv = (int64_t)cf + cb + 3;
+    RCHOL_TRY(sc.get(&lv, nlv));
+    int32_t* flags = reinterpret_cast<int32_t*>(lv);
+    int4 *lvf = lv + 1, *lvb = lvf + cf + 1;
+    RCHOL_TRY(cudaMemsetAsync(flags, 0x7f, sizeof(int4), s));
+    level_table_kernel<<<grid_for(f.npt_f, 256), 256, 0, s>>>(f.npt_f, f.pack_f, f.order_f, levf, f.n, lf0, cf, lvf,
+                                                              flags);
+    level_table_kernel<<<grid_for(f.npt_b, 256), 256, 0, s>>>(f.npt_b, f.pack_b, f.order_b, levb, f.n, 0, cb, lvb,
+                                                              flags + 1);
     RCHOL_TRY(cudaGetLastError());
-    std::vector<int4> h((size_t)lvcap + 1);
-    int32_t hf[2] = {0, 0};
+    std::vector<int4> h((size_t)nlv);
     RCHOL_TRY(cudaMemcpyAsync(h.data(), lv, sizeof(int4) * h.size(), cudaMemcpyDeviceToHost, s));
-    RCHOL_TRY(cudaMemcpyAsync(hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, s));
     RCHOL_TRY(cudaStreamSynchronize(s));
+    const int32_t split_b = h[0].y;
+    const int4 *hf = h.data() + 1, *hb = hf + cf + 1;
     int nlev = 0, stage = 0;
-    for (int l = 0; l < lvcap && l < hf[0]; ++l) {
-        const int ntask = h[l + 1].x - h[l].x, units = h[l + 1].y - h[l].y, rows = h[l + 1].z - h[l].z;
-        if (rows > kHeadMaxRows || ntask > kHeadMaxTasks) break;
-        const int st = std::max(stage, head_stage_bytes(ntask, units, rows, 8));
-        if (head_smem_bytes(h[l + 1].z, st) > kHeadSmem) break;
+    for (int l = 0; l < cb && l < split_b; ++l) {
+        const int ntask = hb[l + 1].x - hb[l].x, units = hb[l + 1].y - hb[l].y, rows = hb[l + 1].z - hb[l].z;
+        if (rows > kHeadMaxRows || ntask > kHeadParts) break;
+        const int st = std::max(stage, head_stage_bytes(ntask, units, rows));
+        if (head_bytes(hb[l + 1].z, st) > kHeadBytes) break;
         stage = st;
         nlev = l + 1;
     }
-    if (nlev < kHeadMinLevels) return cudaSuccess;
-    const int32_t rows = h[nlev].z;
-    const int64_t nslots = (int64_t)h[nlev].y * 32;
-    int32_t* pos = nullptr;
-    RCHOL_TRY(sc.get(&pos, f.n));
-    RCHOL_TRY(ensure(&f.hb_lv, f.cap_hl, (int64_t)kHeadMaxLevels + 1));
-    RCHOL_TRY(ensure(&f.hb_idx, f.cap_hi, std::max<int64_t>(nslots, 32)));
-    invert_order_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(f.n, f.order_b, pos);
-    head_idx_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(nslots, f.pb_idx, pos, rows, f.hb_idx, flags + 1);
-    RCHOL_TRY(cudaGetLastError());
-    RCHOL_TRY(cudaMemcpyAsync(f.hb_lv, lv, sizeof(int4) * ((size_t)nlev + 1), cudaMemcpyDeviceToDevice, s));
-    RCHOL_TRY(cudaMemcpyAsync(&hf[1], flags + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    RCHOL_TRY(cudaStreamSynchronize(s));
-    if (hf[1] != 0) return cudaSuccess;  // not a head after all: leave it empty
-    f.hb_nlev = nlev;
-    f.hb_ntask = h[nlev].x;
-    f.hb_rows = rows;
-    f.hb_stage = stage;
-    return cudaSuccess;
+    if (nlev < kHeadMinLevels) nlev = 0;
+    int nb = nlev;
+    while (nb < cb && hb[nb + 1].x - hb[nb].x <= kNarrowTasks && hb[nb + 1].z <= kNarrowRows) ++nb;
+    int nf = cf;  // first narrow level of the forward table
+    while (nf > 0 && hf[nf].x - hf[nf - 1].x <= kNarrowTasks && hf[cf].z - hf[nf - 1].z <= kNarrowRows) --nf;
+    if (cf - nf >= kNarrowMinLevels) {
+        const int64_t nslots = (int64_t)(hf[cf].y - hf[nf].y) * 32;
+        RCHOL_TRY(ensure(&f.nf_idx, f.cap_nf, std::max<int64_t>(nslots, 32)));
+        f.nf_task = hf[nf].x;
+        f.nf_unit = hf[nf].y;
+        f.nf_pos = hf[nf].z;
+        f.nf_rows = hf[cf].z - hf[nf].z;
+        narrow_idx_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(nslots, f.pf_idx + (int64_t)f.nf_unit * 32, pos_f,
+                                                                f.nf_pos, f.nf_rows, f.nf_idx);
+    }
+    if (nb >= kNarrowMinLevels) {
+        const int64_t nslots = (int64_t)hb[nb].y * 32;
+        int32_t* pos = nullptr;
+        RCHOL_TRY(sc.get(&pos, f.n));
+        RCHOL_TRY(ensure(&f.nb_idx, f.cap_nb, std::max<int64_t>(nslots, 32)));
+        f.nb_task = hb[nb].x;
+        f.nb_rows = hb[nb].z;
+        invert_order_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(f.n, f.order_b, pos);
+        narrow_idx_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(nslots, f.pb_idx, pos, 0, f.nb_rows, f.nb_idx);
+    }
+    // slots per lane of the mean narrow task: stencil factors 2.6 to 4.3, a power-law one 6.6
+    const int64_t units = (f.nf_rows ? hf[cf].y - hf[nf].y : 0) + (f.nb_rows ? hb[nb].y : 0);
+    const int64_t tasks = (f.nf_rows ? hf[cf].x - hf[nf].x : 0) + f.nb_task;
+    f.narrow_long = units > 5 * tasks;
+    if (nlev > 0) {
+        RCHOL_TRY(ensure(&f.hb_lv, f.cap_hl, (int64_t)nlev + 1));
+        RCHOL_TRY(cudaMemcpyAsync(f.hb_lv, lvb, sizeof(int4) * ((size_t)nlev + 1), cudaMemcpyDeviceToDevice, s));
+        f.hb_nlev = nlev;
+        f.hb_ntask = hb[nlev].x;
+        f.hb_rows = hb[nlev].z;
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t build_solve_layouts(DevFactor& f, Scratch& sc, cudaStream_t s) {
@@ -1021,7 +1044,7 @@ cudaError_t build_solve_layouts(DevFactor& f, Scratch& sc, cudaStream_t s) {
 cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bool exact_bwd, bool bwd_head,
                                  double timeout_s, Scratch& sc, cudaStream_t s) {
     if (epl < 1) epl = 1;
-    f.hb_nlev = f.hb_ntask = f.hb_rows = f.hb_stage = 0;
+    clear_narrow(f);
     f.lay_ready = false;
     {
         const bool grow_n = f.cap_n < (int64_t)f.n + 1;
@@ -1039,7 +1062,8 @@ cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bo
         RCHOL_TRY(build_one_schedule(level, f.lc_ptr, f.n, f.depth, 1, epl, sc, f.order_b, &f.tasks_b, f.cap_tb,
                                      &f.ntasks_b, s));
         // reversed forward levels: the backward gate is the dependency of least forward level
-        RCHOL_TRY(build_packs(f, level, level, -1, sc, s));
+        int32_t* pos = nullptr;
+        RCHOL_TRY(build_packs(f, level, level, -1, &pos, sc, s));
         return cudaStreamSynchronize(s);
     }
     // true backward levels, visited in the reversed forward order
@@ -1063,8 +1087,9 @@ cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bo
     f.depth_b = hs[1] + 1;
     RCHOL_TRY(build_one_schedule(levb, f.lc_ptr, f.n, f.depth_b, 0, epl, sc, f.order_b, &f.tasks_b, f.cap_tb,
                                  &f.ntasks_b, s));
-    RCHOL_TRY(build_packs(f, level, levb, 1, sc, s));
-    if (bwd_head) RCHOL_TRY(build_bwd_head(f, levb, sc, s));
+    int32_t* pos_f = nullptr;
+    RCHOL_TRY(build_packs(f, level, levb, 1, &pos_f, sc, s));
+    if (bwd_head) RCHOL_TRY(build_narrow(f, level, levb, pos_f, sc, s));
     return cudaStreamSynchronize(s);
 }
 

@@ -116,7 +116,7 @@ void free_factor(DevFactor& f) {
                   f.lr_val32, f.diag, f.diag32, f.order_f, f.order_b, f.tasks_f, f.tasks_b,
                   f.pack_f, f.pack_b, f.pf_idx, f.pf_val, f.pf_val32, f.pb_idx, f.pb_val, f.pb_val32,
                   f.split_f, f.split_b, f.psum_f, f.psum_b, f.pcount_f, f.pcount_b, f.srow_f, f.srow_b,
-                  f.hb_lv, f.hb_idx, f.sf_ptr, f.sf_idx, f.sf_val, f.sf_val32, f.sb_ptr, f.sb_idx, f.sb_val,
+                  f.hb_lv, f.nf_idx, f.nb_idx, f.sf_ptr, f.sf_idx, f.sf_val, f.sf_val32, f.sb_ptr, f.sb_idx, f.sb_val,
                   f.sb_val32};
     for (void* p : ps) cudaFree(p);
     f = DevFactor();
@@ -833,8 +833,9 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     info.fills = (long long)c64[1];
     info.tail_vertices = std::min<int32_t>(std::max(0, o.tail_vertices), ctx->A.n);
     if (info.tail_vertices > 0) ++info.kernel_launches;
-    // backward head: level table, then (when built) the inverse order and its slab indices
-    if (o.exact_bwd_levels && o.bwd_head) info.kernel_launches += 1 + (f->F.hb_nlev > 0 ? 2 : 0);
+    // narrow levels: both level tables, then (when built) their slab indices
+    if (o.exact_bwd_levels && o.bwd_head)
+        info.kernel_launches += 2 + (f->F.nf_rows > 0 ? 1 : 0) + (f->F.nb_rows > 0 ? 2 : 0);
     f->info = info;
     *out = f;
     return RCHOL_OK;

@@ -236,17 +236,25 @@ struct DevFactor {
             cap_pwb = 0;
     int32_t depth = 0;        // number of levels of the forward solve DAG
     int32_t depth_b = 0;      // levels of the backward schedule
-    // Backward head: the first hb_nlev levels of the backward schedule
-    // (exact levels only), narrow levels of the vertices eliminated last
-    // whose rows depend only on earlier head rows.  One CTA solves them
-    // before the persistent kernel, which then starts at task hb_ntask.
-    // hb_lv[l] = {first task, first slab unit, first position in order_b, 0}
-    // for l <= hb_nlev; hb_idx holds the head's slab slots with every index
-    // replaced by its position in order_b (-1 past a row's end).
-    int32_t hb_nlev = 0, hb_ntask = 0, hb_rows = 0, hb_stage = 0;
+    // Narrow levels: the last levels of the forward schedule (tasks from
+    // nf_task, slab units from nf_unit, positions of order_f from nf_pos,
+    // nf_rows rows) and the first of the backward one (nb_task tasks, nb_rows
+    // rows), solved by one cluster of CTAs whose shared memory holds their
+    // values (exact backward levels only; no rows: none).  nf_idx / nb_idx
+    // hold their slab slots with every index replaced: a row of the range by
+    // its position there, another row j by -1 - j, a slot past the row's end
+    // by INT32_MIN.
+    int32_t nf_task = 0, nf_unit = 0, nf_pos = 0, nf_rows = 0, nb_task = 0, nb_rows = 0;
+    bool narrow_long = false;  // these rows hold many slots per lane
+    int32_t* nf_idx = nullptr;
+    int32_t* nb_idx = nullptr;
+    // The first hb_nlev backward levels (hb_ntask tasks, hb_rows rows): their
+    // r.z terms form one sum of their own, task w of every level in its w-th
+    // part.  hb_lv[l] = {first task, first slab unit, first position in
+    // order_b, 0} for l <= hb_nlev.
+    int32_t hb_nlev = 0, hb_ntask = 0, hb_rows = 0;
     int4* hb_lv = nullptr;
-    int32_t* hb_idx = nullptr;
-    int64_t cap_hl = 0, cap_hi = 0;
+    int64_t cap_hl = 0, cap_nf = 0, cap_nb = 0;
     // allocated capacities (buffers of a released factor are reused)
     int64_t cap_n = 0, cap_nnz = 0, cap_tf = 0, cap_tb = 0, cap_ln = 0, cap_lz = 0;
 };
@@ -283,35 +291,39 @@ inline int auto_sched_epl(int64_t max_row_len) { return max_row_len <= 1024 ? 3 
 // The multi-RHS layouts of a factor (DevFactor::sf_ptr); no-op when built.
 cudaError_t build_solve_layouts(DevFactor& f, Scratch& sc, cudaStream_t s);
 
-// Shared-memory plan of the backward-head kernel: the head holds at most
-// kHeadMaxLevels levels of at most kHeadMaxRows rows and kHeadMaxTasks
-// tasks each; its stages (one level each, kHeadStages in flight) and the
-// per-row arrays fit kHeadSmem.
-constexpr int kHeadThreads = 512;
-constexpr int kHeadStages = 5;
-constexpr int kHeadMaxLevels = 16384;
-// level-table entries the head kernel keeps in shared memory (a ring filled
-// kHeadLvAhead levels ahead)
-constexpr int kHeadLvRing = 16;
-constexpr int kHeadLvAhead = 9;
-constexpr int kHeadMaxRows = 1024;
-// one task per warp of the 16-warp CTA: levels with more tasks than warps
-// took longer in the head kernel than in the persistent one
-constexpr int kHeadMaxTasks = kHeadThreads / 32;
+// Narrow levels of the K = 1 solves: one cluster of kNarrowCtas CTAs solves
+// up to kNarrowRows rows a direction (each CTA's shared memory holds a copy of
+// their values: 208 of the 227 KB), in levels of at most kNarrowTasks tasks;
+// fewer than kNarrowMinLevels such levels stay with the persistent kernels.
+// 128 tasks: half the cluster's warps.  Solve times with 64 / 128 / 256: 256^2
+// grid 7.0 / 6.3 / 6.3 ms, 61x53x47 (iterations only) 12.8 / 11.4 / 11.4, 128^3
+// one apply 1.02 / 1.01 / 1.10.  16 CTAs against 4 and 1: 256^2 6.3 / 7.0 / 7.7
+// ms (each with the levels that suit it); small systems lose 3% to 4 CTAs.
+constexpr int kNarrowCtas = 16;
+constexpr int kNarrowRows = 26 * 1024;
+constexpr int kNarrowTasks = 128;
+constexpr int kNarrowMinLevels = 8;
+constexpr int kNarrowMaxLevels = 16384;
+
+// The rows whose r.z terms are summed apart (DevFactor::hb_nlev): the
+// backward levels from the first while each holds at most kHeadMaxRows rows,
+// kHeadParts tasks and no part task, and head_bytes of them stays within
+// kHeadBytes.  The sum's grouping, and so the last bits of every iterate,
+// follows these limits.
+constexpr int kHeadParts = 16;
 constexpr int kHeadMinLevels = 8;
-constexpr int kHeadSmem = 220 * 1024;
-// Bytes of one head stage (a level's descriptors, slab slots and row
-// scalars) for value size vb, each part 16-byte aligned.
-inline int head_stage_bytes(int ntask, int units, int rows, int vb) {
+constexpr int kHeadMaxRows = 1024;
+constexpr int kHeadBytes = 220 * 1024;
+inline int head_stage_bytes(int ntask, int units, int rows) {
     auto al = [](int x) { return (x + 15) & ~15; };
-    return 16 * ntask + 128 * units + 32 * vb * units + 2 * al(8 * rows) + al(vb * rows);
+    return 16 * ntask + 384 * units + 3 * al(8 * rows);
 }
-// Dynamic shared memory of the head kernel: row ids and z values of every
-// head row, the level-table ring and the stages.
-inline int head_smem_bytes(int rows, int stage) {
-    return ((4 * rows + 15) & ~15) + ((8 * rows + 15) & ~15) + 16 * kHeadLvRing + kHeadStages * stage;
+inline int head_bytes(int rows, int stage) {
+    return ((4 * rows + 15) & ~15) + ((8 * rows + 15) & ~15) + 256 + 5 * stage;
 }
-// bwd_head (exact levels only): build the backward head (DevFactor::hb_nlev).
+
+// bwd_head (exact levels only): give the narrow levels to the cluster kernel
+// (DevFactor::nf_rows).
 cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bool exact_bwd, bool bwd_head,
                                  double timeout_s, Scratch& sc, cudaStream_t s);
 

@@ -9,6 +9,8 @@
 //                (A p computed as A z + beta A p_old: no separate p pass)
 //   fwd          x += alpha p, r -= alpha q, (r.r); y = L^-1 r   sync-free
 //   bwd          z = L^-T D^+ y, (r.z) -> beta, stop test        sync-free
+// and, for one right-hand side, a fourth between the last two: the narrow
+// levels of both sweeps on one cluster (narrow_kernel).
 // The triangular solves are persistent kernels over the resident grid: each
 // row group waits for the rows it depends on by polling their values, which
 // start as a "pending" NaN bit pattern (no separate ready flags, no level
@@ -103,11 +105,17 @@ struct SolveArgs {
     int32_t* pcount_b;
     const int32_t* __restrict__ srow_b;
     int32_t nsplit_b;
-    // backward head (see DevFactor::hb_nlev); the persistent backward
-    // kernel starts at task hb_ntask (0: no head)
+    // narrow levels of both directions (see DevFactor::nf_rows): the forward
+    // tasks from nf_task on and the backward tasks before nb_task are
+    // narrow_kernel's; the r.z terms of the first hb_nlev backward levels
+    // (hb_ntask tasks) are added there too, those of the others by
+    // bwd_pack_kernel (nf_rows = nb_rows = 0: every task is a pack kernel's)
+    const int32_t* __restrict__ nf_idx;
+    const int32_t* __restrict__ nb_idx;
     const int4* __restrict__ hb_lv;
-    const int32_t* __restrict__ hb_idx;
-    int32_t hb_nlev, hb_ntask, hb_rows, hb_stage;
+    int32_t nf_task, nf_unit, nf_pos, nf_rows;
+    int32_t nb_task, nb_rows, n_long;
+    int32_t hb_nlev, hb_ntask;
     // vectors (n x K row-major)
     const double* __restrict__ b;
     double* x;
@@ -1049,10 +1057,12 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) fwd_pack_kernel(Solve
     double acc[1] = {0.0};
     const unsigned long long t0 = global_timer_ns();
     bool ok = true;
+    const int32_t tend = a.nf_rows > 0 ? a.nf_task : a.ntasks_f;
     PackLane<TV> cur, nxt;
-    if (warp < a.ntasks_f) pack_load(cur, a.pack_f[warp], lane, a.order_f, a.pf_idx, pval);
-    int4 dn = warp + nwarps < a.ntasks_f ? a.pack_f[warp + nwarps] : make_int4(0, 0, 0, 0);
-    for (int64_t t = warp; t < a.ntasks_f && ok; t += nwarps) {
+    if (warp < tend) pack_load(cur, a.pack_f[warp], lane, a.order_f, a.pf_idx, pval);
+    int4 dn = warp + nwarps < tend ? a.pack_f[warp + nwarps] : make_int4(0, 0, 0, 0);
+    int64_t t = warp;
+    for (; t < tend && ok; t += nwarps) {
         const int cls = (cur.d.z >> 8) & 7, cnt = cur.d.z & 0xff;
         const int G = 1 << cls;
         const bool lead = (lane >> cls) < cnt && (lane & (G - 1)) == 0;
@@ -1074,8 +1084,8 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) fwd_pack_kernel(Solve
             }
             if (a.z) a.z[i] = pending_value();
         }
-        if (t + nwarps < a.ntasks_f) pack_load(nxt, dn, lane, a.order_f, a.pf_idx, pval);
-        if (t + 2 * nwarps < a.ntasks_f) dn = a.pack_f[t + 2 * nwarps];
+        if (t + nwarps < tend) pack_load(nxt, dn, lane, a.order_f, a.pf_idx, pval);
+        if (t + 2 * nwarps < tend) dn = a.pack_f[t + 2 * nwarps];
         double sum = pack_dot<TV>(cur, lane, G, a.pf_idx, pval, a.y, t0, a.timeout_ns, &a.sc->status, ok, a.poll_ns);
         sum = group_sum(sum, G);
         if (lead && !part) st_relaxed_f64(a.y + i, ri - sum);
@@ -1093,6 +1103,36 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) fwd_pack_kernel(Solve
         }
         ok = __all_sync(kFull, ok);
         cur = nxt;
+    }
+    // the narrow levels' tasks: their rows' share of the x / r update only,
+    // task by task as above so that r.r keeps its grouping; the next task's
+    // descriptor and row are in flight meanwhile
+    if (t < a.ntasks_f && ok) {
+        int4 d = a.pack_f[t];
+        int4 e = t + nwarps < a.ntasks_f ? a.pack_f[t + nwarps] : make_int4(0, 0, 0, 0);
+        int32_t i = (lane >> ((d.z >> 8) & 7)) < (d.z & 0xff) ? a.order_f[d.x + (lane >> ((d.z >> 8) & 7))] : 0;
+        for (; t < a.ntasks_f; t += nwarps) {
+            const int cls = (d.z >> 8) & 7;
+            const bool lead = (lane >> cls) < (d.z & 0xff) && (lane & ((1 << cls) - 1)) == 0;
+            const int ipart = (d.z >> 11) & 1 ? d.z >> 12 : 0;
+            const int ecls = (e.z >> 8) & 7;
+            const int32_t in = (lane >> ecls) < (e.z & 0xff) ? a.order_f[e.x + (lane >> ecls)] : 0;
+            const int4 e2 = t + 2 * nwarps < a.ntasks_f ? a.pack_f[t + 2 * nwarps] : make_int4(0, 0, 0, 0);
+            if (lead && ipart == 0) {
+                if (a.update) {
+                    double ri = a.r[i];
+                    const double xi = a.x[i], pi = a.p[i], qi = a.q[i];
+                    a.x[i] = xi + alpha * pi;
+                    ri = ri - alpha * qi;
+                    a.r[i] = ri;
+                    acc[0] += ri * ri;
+                }
+                if (a.z) a.z[i] = pending_value();
+            }
+            d = e;
+            e = e2;
+            i = in;
+        }
     }
     if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) a.sc->done = 1;
@@ -1122,8 +1162,26 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) bwd_pack_kernel(Solve
     const unsigned long long t0 = global_timer_ns();
     bool ok = true;
     PackLane<TV> cur, nxt;
-    // the head's tasks were solved by bwd_head_kernel
-    const int64_t tb = a.hb_ntask + warp;
+    // tasks before nb_task were solved by narrow_kernel, which also added the
+    // r.z terms of the first hb_ntask; the others' terms are added here, task
+    // by task as if they ran here, so that r.z keeps its grouping
+    int64_t tb = a.hb_ntask + warp;
+    if (tb < a.nb_task) {
+        int4 d = a.pack_b[tb];
+        int4 e = tb + nwarps < a.nb_task ? a.pack_b[tb + nwarps] : make_int4(0, 0, 0, 0);
+        int32_t j = (lane >> ((d.z >> 8) & 7)) < (d.z & 0xff) ? a.order_b[d.x + (lane >> ((d.z >> 8) & 7))] : 0;
+        for (; tb < a.nb_task; tb += nwarps) {
+            const int cls = (d.z >> 8) & 7;
+            const bool lead = (lane >> cls) < (d.z & 0xff) && (lane & ((1 << cls) - 1)) == 0;
+            const int ecls = (e.z >> 8) & 7;
+            const int32_t jn = (lane >> ecls) < (e.z & 0xff) ? a.order_b[e.x + (lane >> ecls)] : 0;
+            const int4 e2 = tb + 2 * nwarps < a.nb_task ? a.pack_b[tb + 2 * nwarps] : make_int4(0, 0, 0, 0);
+            if (a.reduce && lead && !((d.z >> 11) & 1)) acc[0] += a.r[j] * ld_relaxed_f64(a.z + j);
+            d = e;
+            e = e2;
+            j = jn;
+        }
+    }
     if (tb < a.ntasks_b) pack_load(cur, a.pack_b[tb], lane, a.order_b, a.pb_idx, pval);
     int4 dn = tb + nwarps < a.ntasks_b ? a.pack_b[tb + nwarps] : make_int4(0, 0, 0, 0);
     for (int64_t t = tb; t < a.ntasks_b && ok; t += nwarps) {
@@ -1187,179 +1245,343 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) bwd_pack_kernel(Solve
 }
 
 // ---------------------------------------------------------------------------
-// Backward head: z for the rows of the first hb_nlev backward levels, solved
-// by one CTA level by level.  These levels are narrow (the vertices
-// eliminated last) and every dependency of a head row is an earlier head
-// row, so the z values live in shared memory and a level costs one CTA
-// barrier instead of a store -> poll hop between SMs.  Each level's task
-// descriptors and slab slots (contiguous ranges) and its rows' y, r and D
-// (gathers) are staged by cp.async kHeadStages - 1 levels ahead.  A lane's
-// products are added in slot order and a row's lanes by the same shuffle
-// tree as bwd_pack_kernel, so z is the persistent kernel's bit for bit;
-// r.z over the head goes to sc->hrz for the backward kernel's reduction.
+// Narrow levels: y for the last levels of the forward schedule, then z for
+// the first of the backward one, by one cluster of kNarrowCtas CTAs.  These
+// levels hold few rows (the vertices eliminated last), so between SMs they
+// cost a store -> poll hop through L2 each.  Here every CTA keeps a copy of
+// the levels' values in its shared memory, pending until known: a row's lanes
+// store the value into all copies (distributed shared memory), and a wait
+// polls the CTA's own copy.  Warps take the tasks in schedule order, so every
+// dependency sits in an earlier task.  A task's slots come in chunks,
+// several in flight per warp (a warp's chunks of successive tasks form one
+// stream): index and value loads first, then, a chunk or two ahead of use, the values of rows outside the range (final, from
+// global memory) and the row's own scalars.  A lane's products are added in
+// slot order and a row's lanes by the shuffle tree of the pack kernels, so y
+// and z equal theirs bit for bit.
+// What bounds it is the latency of one row's chain (see the value, re-read the
+// slots, add, shuffle, store to the other CTAs: about 0.9 us a level down to
+// 0.5 on one CTA, where a store between CTAs alone takes 374 cycles), so the waits
+// and sums are free of data-dependent branches; the persistent kernels spend
+// 1.2 us a level.  Per solve iteration, both sweeps: 2867-vertex grid 114 -> 74
+// us, 256^2 178 -> 137, 61x53x47 530 -> 400, power-law (100k vertices) 3.0 -> 2.5
+// ms; one 128^3 apply (FP32) 1.08 -> 0.99 ms.
+// With reduce, CTA 0 adds the r.z terms of the first hb_nlev backward levels
+// (see DevFactor::hb_nlev) while the other CTAs solve.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+// Form of the kernel: kM slots a lane and chunk, kBufs chunks in flight a
+// warp, values outside the range fetched kLead chunks ahead.  Rows of a few
+// slots want the many warps of NarrowShort (61x53x47 grid, 28 iterations: 11.0
+// ms against 12.2 with NarrowLong); rows of many chunks are a serial chain
+// of fetches without NarrowLong's deeper stream (power-law, 100k vertices, 12
+// iterations: 42.4 -> 33.1 ms).
+struct NarrowShort {
+    static constexpr int kM = 4, kBufs = 3, kLead = 1, kThreads = 512;
+};
+struct NarrowLong {
+    static constexpr int kM = 8, kBufs = 4, kLead = 2, kThreads = 256;
+};
+constexpr int kRzWarps = 8;  // of CTA 0, when it adds r.z terms
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
 }
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+// all CTAs of the cluster, with release / acquire of what was written before
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+__device__ __forceinline__ double ld_copy(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.cluster.shared::cta.f64 %0, [%1];"
+                 : "=d"(v)
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
+    return v;
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// v to the same address in CTA `rank` of the cluster
+__device__ __forceinline__ void st_copy(double* p, unsigned rank, double v) {
+    if (kNarrowCtas == 1) {
+        *reinterpret_cast<volatile double*>(p) = v;
+        return;
+    }
+    unsigned d;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(d), "d"(v) : "memory");
 }
 
-// Byte offsets of one level's stage (head_stage_bytes with the value size of TV).
-struct HeadLevel {
-    int ntask, units, rows, o_idx, o_val, o_y, o_r, o_d;
+template <typename TV, int kM>
+struct NarrowChunk {
+    int32_t pos;   // the task's first position
+    int32_t dz;    // descriptor words z and w
+    int32_t dw;
+    int32_t k0;    // first slot
+    int32_t row;
+    int32_t idx[kM];
+    TV val[kM];
+    double out[kM];  // values of rows outside the range
+    double t, dj;          // the row's right-hand side (backward: before the division by dj)
 };
 
-template <typename TV>
-__device__ __forceinline__ HeadLevel head_level(const int4& lo, const int4& hi) {
-    HeadLevel L;
-    L.ntask = hi.x - lo.x;
-    L.units = hi.y - lo.y;
-    L.rows = hi.z - lo.z;
-    L.o_idx = 16 * L.ntask;
-    L.o_val = L.o_idx + 128 * L.units;
-    L.o_y = L.o_val + 32 * (int)sizeof(TV) * L.units;
-    L.o_r = L.o_y + ((8 * L.rows + 15) & ~15);
-    L.o_d = L.o_r + ((8 * L.rows + 15) & ~15);
-    return L;
-}
-
-// Copies of level l into its stage, spread over threads tid of nthr; lv is
-// the shared ring of level-table entries (entry x in slot x % kHeadLvRing).
-template <typename TV>
-__device__ __forceinline__ void head_issue(const SolveArgs& a, const int4* lv, const int32_t* rows_s, int l,
-                                           char* buf, int tid, int nthr) {
-    const int4 lo = lv[l & (kHeadLvRing - 1)], hi = lv[(l + 1) & (kHeadLvRing - 1)];
-    const HeadLevel L = head_level<TV>(lo, hi);
-    for (int i = tid; i < L.ntask; i += nthr) cp_async16(buf + 16 * i, a.pack_b + lo.x + i);
-    const char* gi = reinterpret_cast<const char*>(a.hb_idx + (size_t)lo.y * 32);
-    for (int i = tid; i < 8 * L.units; i += nthr) cp_async16(buf + L.o_idx + 16 * i, gi + 16 * i);
-    const char* gv = reinterpret_cast<const char*>(a.pb_val) + (size_t)lo.y * 32 * sizeof(TV);
-    for (int i = tid; i < 2 * (int)sizeof(TV) * L.units; i += nthr) cp_async16(buf + L.o_val + 16 * i, gv + 16 * i);
-    const TV* dv = reinterpret_cast<const TV*>(a.diag);
-    for (int i = tid; i < L.rows; i += nthr) {
-        const int32_t j = rows_s[lo.z + i];
-        cp_async8(buf + L.o_y + 8 * i, a.y + j);
-        if (a.reduce) cp_async8(buf + L.o_r + 8 * i, a.r + j);
-        if (sizeof(TV) == 4) cp_async4(buf + L.o_d + 4 * i, dv + j);
-        else cp_async8(buf + L.o_d + 8 * i, dv + j);
-    }
-}
-
-template <typename TV>
-__global__ void __launch_bounds__(kHeadThreads, 1) bwd_head_kernel(SolveArgs a) {
-    if ((a.reduce || a.seg) && ld_relaxed(&a.sc->done)) return;
-    extern __shared__ __align__(16) char hsm[];
-    const int R = a.hb_rows, nlev = a.hb_nlev;
-    // layout of head_smem_bytes: row ids | z | level-table ring | stages
-    int32_t* rows_s = reinterpret_cast<int32_t*>(hsm);
-    double* zs = reinterpret_cast<double*>(hsm + ((4 * R + 15) & ~15));
-    int4* lv = reinterpret_cast<int4*>(hsm + ((4 * R + 15) & ~15) + ((8 * R + 15) & ~15));
-    char* ring = reinterpret_cast<char*>(lv + kHeadLvRing);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < R; i += kHeadThreads) rows_s[i] = a.order_b[i];
-    // entries 0 .. kHeadLvAhead - 1 now; entry l + kHeadLvAhead rides in the
-    // commit group of level l, so it has landed by level l + 4 (whose issue
-    // reads entries up to l + kHeadLvAhead)
-    for (int i = tid; i < kHeadLvAhead && i <= nlev; i += kHeadThreads) lv[i] = a.hb_lv[i];
-    __syncthreads();
-    constexpr int NW = kHeadThreads / 32;
-    // levels 0 .. kHeadStages - 2 in flight; one commit group per level
-    for (int l = 0; l < kHeadStages - 1; ++l) {
-        if (l < nlev) head_issue<TV>(a, lv, rows_s, l, ring + (size_t)l * a.hb_stage, tid, kHeadThreads);
-        cp_async_commit();
-    }
-    double acc = 0.0;
-    for (int l = 0; l < nlev; ++l) {
-        // level l's copies have landed (this thread's, then everyone's), and
-        // every warp is done with level l - 1, whose stage is refilled with
-        // level l + kHeadStages - 1 by the warps that hold no task of level l
-        // (all warps when every warp holds one)
-        cp_async_wait<kHeadStages - 2>();
-        __syncthreads();
-        const char* buf = ring + (size_t)(l % kHeadStages) * a.hb_stage;
-        const int4 lo = lv[l & (kHeadLvRing - 1)];
-        const HeadLevel L = head_level<TV>(lo, lv[(l + 1) & (kHeadLvRing - 1)]);
-        {
-            const int lf = l + kHeadStages - 1;
-            const int busy = L.ntask < NW ? L.ntask : 0;
-            if (lf < nlev && warp >= busy)
-                head_issue<TV>(a, lv, rows_s, lf, ring + (size_t)(lf % kHeadStages) * a.hb_stage, tid - 32 * busy,
-                               kHeadThreads - 32 * busy);
-            const int le = l + kHeadLvAhead;
-            if (tid == kHeadThreads - 1 && le <= nlev) cp_async16(lv + (le & (kHeadLvRing - 1)), a.hb_lv + le);
-            cp_async_commit();
-        }
-        const int4* desc = reinterpret_cast<const int4*>(buf);
-        const int32_t* idx_s = reinterpret_cast<const int32_t*>(buf + L.o_idx);
-        const TV* val_s = reinterpret_cast<const TV*>(buf + L.o_val);
-        const double* y_s = reinterpret_cast<const double*>(buf + L.o_y);
-        const double* r_s = reinterpret_cast<const double*>(buf + L.o_r);
-        const TV* d_s = reinterpret_cast<const TV*>(buf + L.o_d);
-        for (int ti = warp; ti < L.ntask; ti += NW) {
-            const int4 d = desc[ti];
-            const int cls = (d.z >> 8) & 7, cnt = d.z & 0xff, m = d.w & 0xff;
-            const int G = 1 << cls;
-            const int ub = d.y - lo.y;
-            double sum = 0.0;
-            int k = 0;
-            for (; k + 4 <= m; k += 4) {  // four slots' loads in flight, added in slot order
-                const int sl = (ub + k) * 32 + lane;
-                const int32_t i0 = idx_s[sl], i1 = idx_s[sl + 32], i2 = idx_s[sl + 64], i3 = idx_s[sl + 96];
-                const double w0 = to_d(val_s[sl]), w1 = to_d(val_s[sl + 32]), w2 = to_d(val_s[sl + 64]),
-                             w3 = to_d(val_s[sl + 96]);
-                const double v0 = i0 >= 0 ? zs[i0] : 0.0, v1 = i1 >= 0 ? zs[i1] : 0.0;
-                const double v2 = i2 >= 0 ? zs[i2] : 0.0, v3 = i3 >= 0 ? zs[i3] : 0.0;
-                sum += w0 * v0;
-                sum += w1 * v1;
-                sum += w2 * v2;
-                sum += w3 * v3;
-            }
-            for (; k < m; ++k) {
-                const int sl = (ub + k) * 32 + lane;
-                const int32_t ix = idx_s[sl];
-                const double v = ix >= 0 ? zs[ix] : 0.0;
-                sum += to_d(val_s[sl]) * v;
-            }
-            sum = group_sum(sum, G);
-            const int qrow = lane >> cls;
-            if (qrow < cnt && (lane & (G - 1)) == 0) {
-                const int pos = d.x + qrow;
-                const int rl = pos - lo.z;
-                const double dj = to_d(d_s[rl]);
-                double tj = y_s[rl];
-                if (dj != 0.0) tj = tj / dj;
-                const double zj = tj - sum;
-                zs[pos] = zj;
-                a.z[rows_s[pos]] = zj;
-                if (a.reduce) acc += r_s[rl] * zj;
-            }
-        }
-    }
-    cp_async_wait<0>();
-    if (!a.reduce) return;
-    // r.z over the head: warps in order, lanes by a fixed tree
-    __shared__ double red[kHeadThreads / 32];
+// One direction's narrow tasks [t0, t1): warp `id` of `nw` takes t0 + id,
+// t0 + id + nw, ...; slab units are relative to u0, positions to p0.
+template <typename TV, typename Form, bool FWD>
+__device__ bool narrow_tasks(const SolveArgs& a, double* copy, int id, int nw, int32_t t0, int32_t t1, int32_t u0,
+                             int32_t p0, unsigned long long start) {
+    constexpr int kM = Form::kM, kBufs = Form::kBufs;
+    const int lane = threadIdx.x & 31;
+    const int4* __restrict__ pack = FWD ? a.pack_f : a.pack_b;
+    const int32_t* __restrict__ order = FWD ? a.order_f : a.order_b;
+    const int32_t* __restrict__ nidx = FWD ? a.nf_idx : a.nb_idx;
+    const TV* __restrict__ nval =
+        reinterpret_cast<const TV*>(FWD ? a.pf_val : a.pb_val) + (size_t)u0 * 32;
+    const TV* __restrict__ dv = reinterpret_cast<const TV*>(a.diag);
+    double* vec = FWD ? a.y : a.z;
+    // the loader's place in the warp's stream of chunks
+    int32_t lt = t0 + id, lk = 0;
+    int4 ld = lt < t1 ? pack[lt] : make_int4(0, 0, 0, 0);
+    int4 ldn = lt + nw < t1 ? pack[lt + nw] : make_int4(0, 0, 0, 0);
+    NarrowChunk<TV, kM> buf[kBufs];
+    auto load = [&](NarrowChunk<TV, kM>& c) {
+        c.pos = ld.x;
+        c.dz = ld.z;
+        c.dw = ld.w;
+        c.k0 = lk;
+        const int m = ld.w & 0xff;
+        const int cls = (ld.z >> 8) & 7;
+        c.row = (lane >> cls) < (ld.z & 0xff) ? order[ld.x + (lane >> cls)] : -1;
+        const size_t o = ((size_t)(ld.y - u0) + lk) * 32 + lane;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-    if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (tid == 0) {
+        for (int k = 0; k < kM; ++k) {
+            c.idx[k] = INT_MIN;
+            c.val[k] = TV(0);
+            if (lk + k < m) {
+                c.idx[k] = nidx[o + 32 * k];
+                c.val[k] = nval[o + 32 * k];
+            }
+        }
+        lk += kM;
+        if (lk >= m) {
+            lk = 0;
+            lt = lt < t1 ? lt + nw : lt;
+            ld = ldn;
+            ldn = lt + nw < t1 && lt < t1 ? pack[lt + nw] : make_int4(0, 0, 0, 0);
+        }
+    };
+    auto gather = [&](NarrowChunk<TV, kM>& c) {
+#pragma unroll
+        for (int k = 0; k < kM; ++k) {
+            c.out[k] = 0.0;
+            if (FWD && c.idx[k] < 0 && c.idx[k] != INT_MIN) c.out[k] = ld_relaxed_f64(vec + (-1 - c.idx[k]));
+        }
+        c.t = 0.0;
+        c.dj = 0.0;
+        if (c.row >= 0 && c.k0 + kM >= (c.dw & 0xff)) {
+            if (FWD) {
+                c.t = a.r[c.row];
+            } else {
+                c.t = ld_relaxed_f64(a.y + c.row);
+                c.dj = to_d(dv[c.row]);
+            }
+        }
+    };
+#pragma unroll
+    for (int b = 0; b < kBufs; ++b) load(buf[b]);
+    gather(buf[0]);
+    if (Form::kLead > 1) gather(buf[1]);
+    double sum = 0.0;
+    int32_t t = t0 + id;
+    while (t < t1) {
+#pragma unroll
+        for (int b = 0; b < kBufs; ++b) {
+            NarrowChunk<TV, kM>& c = buf[b];
+            gather(buf[(b + Form::kLead) % kBufs]);
+            if (t >= t1) break;
+            const int cls = (c.dz >> 8) & 7, cnt = c.dz & 0xff, m = c.dw & 0xff;
+            const int G = 1 << cls, g = lane & (G - 1);
+            double tj = c.t;
+            if (!FWD && c.dj != 0.0) tj = tj / c.dj;
+            asm volatile("" : "+d"(tj));  // the division stays ahead of the waits
+            if (c.k0 == 0) sum = 0.0;
+            // Waits and sums hold no data-dependent branch: from the last
+            // dependency's arrival to the store every instruction counts.
+            // The row's gate (its last dependency) alone first, then all slots.
+            unsigned spins = 0;
+            bool late = false;
+            if (c.k0 == 0) {
+                const bool gate = g == 0 & c.idx[0] >= 0;
+                const double* gp = copy + max(c.idx[0], 0);
+                while (__any_sync(kFull, gate & is_pending(ld_copy(gp)))) {
+                    if ((++spins & 255u) == 0 && __any_sync(kFull, timed_out(start, a.timeout_ns))) {
+                        late = true;
+                        break;
+                    }
+                }
+            }
+            double v[kM];
+            while (!late) {
+                bool pend = false;
+#pragma unroll
+                for (int k = 0; k < kM; ++k) v[k] = ld_copy(copy + max(c.idx[k], 0));
+#pragma unroll
+                for (int k = 0; k < kM; ++k) pend |= c.idx[k] >= 0 & is_pending(v[k]);
+                if (!__any_sync(kFull, pend)) break;
+                if ((++spins & 255u) == 0 && __any_sync(kFull, timed_out(start, a.timeout_ns))) late = true;
+            }
+            if (late) {
+                if (lane == 0) raise_error(&a.sc->status, kDevTimeout);
+                return false;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) sum += to_d(c.val[k]) * (c.idx[k] >= 0 ? v[k] : c.out[k]);
+            if (kM > 4 && m - c.k0 > 4) {
+#pragma unroll
+                for (int k = 4; k < kM; ++k) sum += to_d(c.val[k]) * (c.idx[k] >= 0 ? v[k] : c.out[k]);
+            }
+            if (c.k0 + kM >= m) {
+                switch (cls) {
+                    case 5: sum += __shfl_xor_sync(kFull, sum, 16); [[fallthrough]];
+                    case 4: sum += __shfl_xor_sync(kFull, sum, 8); [[fallthrough]];
+                    case 3: sum += __shfl_xor_sync(kFull, sum, 4); [[fallthrough]];
+                    case 2: sum += __shfl_xor_sync(kFull, sum, 2); [[fallthrough]];
+                    case 1: sum += __shfl_xor_sync(kFull, sum, 1); [[fallthrough]];
+                    default: break;
+                }
+                const bool in = (lane >> cls) < cnt;
+                double* at = copy + (c.pos - p0) + (lane >> cls);
+                if (!((c.dz >> 11) & 1)) {
+                    const double r = tj - sum;
+                    if (in) {
+                        for (int q = g; q < kNarrowCtas; q += G) st_copy(at, q, r);
+                        if (g == 0) st_relaxed_f64(vec + c.row, r);
+                    }
+                } else if (in && g == 0) {
+                    // partial sum; the last part to finish adds them in part order
+                    const int2 sp = (FWD ? a.split_f : a.split_b)[t];
+                    double* psum = FWD ? a.psum_f : a.psum_b;
+                    int32_t* pcount = FWD ? a.pcount_f : a.pcount_b;
+                    const int np = c.dw >> 8;
+                    psum[sp.y + (c.dz >> 12)] = sum;
+                    if (atom_add_acq_rel(pcount + sp.x, 1) == np - 1) {
+                        double tot = 0.0;
+                        for (int q = 0; q < np; ++q) tot += ld_relaxed_f64(psum + sp.y + q);
+                        const double r = tj - tot;
+                        for (int q = 0; q < kNarrowCtas; ++q) st_copy(at, q, r);
+                        st_relaxed_f64(vec + c.row, r);
+                        pcount[sp.x] = 0;
+                    }
+                }
+                __syncwarp();
+                t += nw;
+            }
+            load(c);
+        }
+    }
+    return true;
+}
+
+// r.z over the first hb_nlev backward levels by the last 8 warps of a CTA: warp
+// w adds the terms of tasks w and w + 8 of every level in level order, lanes
+// by a fixed tree, then the 16 sums in task order.  Four levels' scalars are
+// in flight before their z values are polled.
+template <int kThreads>
+__device__ bool narrow_rz(const SolveArgs& a, const double* copy, unsigned long long start) {
+    constexpr int NP = kHeadParts / kRzWarps, U = 4;
+    __shared__ double red[kHeadParts];
+    const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) - (kThreads / 32 - kRzWarps);
+    double acc[NP] = {};
+    bool ok = true;
+    for (int l0 = 0; l0 < a.hb_nlev && ok; l0 += U) {
+        int32_t first[U + 1];
+#pragma unroll
+        for (int u = 0; u <= U; ++u) first[u] = a.hb_lv[min(l0 + u, a.hb_nlev)].x;
+        int32_t pos[U][NP];
+        double r[U][NP];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const int w = warp + p * kRzWarps;
+                pos[u][p] = -1;
+                if (first[u] + w < first[u + 1]) {
+                    const int4 d = a.pack_b[first[u] + w];
+                    const int cls = (d.z >> 8) & 7;
+                    if ((lane >> cls) < (d.z & 0xff) && (lane & ((1 << cls) - 1)) == 0) pos[u][p] = d.x + (lane >> cls);
+                }
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) r[u][p] = pos[u][p] >= 0 ? a.r[a.order_b[pos[u][p]]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                if (pos[u][p] >= 0) {
+                    double v = ld_copy(copy + pos[u][p]);
+                    unsigned spins = 0;
+                    while (is_pending(v) && ok) {
+                        v = ld_copy(copy + pos[u][p]);
+                        if ((++spins & 255u) == 0 && timed_out(start, a.timeout_ns)) {
+                            raise_error(&a.sc->status, kDevTimeout);
+                            ok = false;
+                        }
+                    }
+                    acc[p] += r[u][p] * v;
+                }
+        ok = __all_sync(kFull, ok);
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[p] += __shfl_xor_sync(kFull, acc[p], o);
+        if (lane == 0) red[warp + p * kRzWarps] = acc[p];
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kRzWarps) : "memory");
+    if (warp == 0 && lane == 0) {
         double t = 0.0;
-        for (int w = 0; w < kHeadThreads / 32; ++w) t += red[w];
+        for (int w = 0; w < kHeadParts; ++w) t += red[w];
         a.sc->hrz = t;
     }
+    return ok;
+}
+
+template <typename TV, typename Form>
+__global__ void __launch_bounds__(Form::kThreads, 1) narrow_kernel(SolveArgs a) {
+    // the same answer in every CTA: done is set below only after a barrier
+    // that all of them pass
+    if ((a.reduce || a.seg) && ld_relaxed(&a.sc->done)) return;
+    extern __shared__ __align__(16) double copy[];
+    const int rank = (int)cluster_rank(), warp = threadIdx.x >> 5;
+    constexpr int kThreads = Form::kThreads, NW = kThreads / 32;
+    const unsigned long long start = global_timer_ns();
+    bool ok = true;
+    if (a.nf_rows > 0) {
+        for (int i = threadIdx.x; i < a.nf_rows; i += kThreads) copy[i] = pending_value();
+        cluster_sync();
+        ok = narrow_tasks<TV, Form, true>(a, copy, warp * kNarrowCtas + rank, NW * kNarrowCtas, a.nf_task, a.ntasks_f,
+                                    a.nf_unit, a.nf_pos, start);
+        __syncwarp();
+        cluster_sync();  // every store into this copy has landed, and y is visible
+    }
+    if (a.nb_rows > 0) {
+        for (int i = threadIdx.x; i < a.nb_rows; i += kThreads) copy[i] = pending_value();
+        cluster_sync();
+        const bool rz = a.reduce && a.hb_nlev > 0;
+        constexpr int W0 = NW - kRzWarps;  // warps of CTA 0 that solve
+        if (rz && rank == 0 && warp >= W0) {
+            ok &= narrow_rz<kThreads>(a, copy, start);
+        } else if (ok) {
+            const int id = rz && warp >= W0 ? W0 * kNarrowCtas + (warp - W0) * (kNarrowCtas - 1) + rank - 1
+                                            : warp * kNarrowCtas + rank;
+            ok = narrow_tasks<TV, Form, false>(a, copy, id, NW * kNarrowCtas - (rz ? kRzWarps : 0), 0, a.nb_task, 0, 0,
+                                         start);
+        }
+        __syncwarp();
+        cluster_sync();  // no CTA leaves while stores into its copy may be on their way
+    }
+    if (!ok && (threadIdx.x & 31) == 0) a.sc->done = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1469,6 +1691,56 @@ cudaError_t launch_coresident(const void* fn, int grid, void** params, cudaStrea
     return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
+// The narrow levels (nothing to do without any): one cluster.
+template <typename TV>
+cudaError_t launch_narrow(SolveArgs& a, cudaStream_t s) {
+    if (a.nf_rows == 0 && a.nb_rows == 0) return cudaSuccess;
+    const void* fn =
+        a.n_long ? (const void*)narrow_kernel<TV, NarrowLong> : (const void*)narrow_kernel<TV, NarrowShort>;
+    void* params[] = {&a};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kNarrowCtas);
+    cfg.blockDim = dim3(a.n_long ? NarrowLong::kThreads : NarrowShort::kThreads);
+    cfg.dynamicSmemBytes = sizeof(double) * (size_t)std::max(a.nf_rows, a.nb_rows);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kNarrowCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, params);
+}
+
+template <typename TV>
+cudaError_t narrow_attributes() {
+    const void* fns[2] = {(const void*)narrow_kernel<TV, NarrowLong>, (const void*)narrow_kernel<TV, NarrowShort>};
+    cudaError_t e = cudaSuccess;
+    for (const void* fn : fns) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(double) * kNarrowRows);
+        if (e == cudaSuccess && kNarrowCtas > 8)
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    return e;
+}
+
+void set_narrow(SolveArgs& a, const DevFactor& F) {
+    a.nf_idx = F.nf_idx;
+    a.nb_idx = F.nb_idx;
+    a.nf_task = F.nf_task;
+    a.nf_unit = F.nf_unit;
+    a.nf_pos = F.nf_pos;
+    a.nf_rows = F.nf_rows;
+    a.nb_task = F.nb_task;
+    a.nb_rows = F.nb_rows;
+    a.n_long = F.narrow_long ? 1 : 0;
+    a.hb_lv = F.hb_lv;
+    a.hb_nlev = F.hb_nlev;
+    a.hb_ntask = F.hb_ntask;
+}
+
 template <typename Arg>
 cudaError_t launch_coresident(const void* fn, int grid, Arg& a, cudaStream_t s) {
     void* params[] = {&a};
@@ -1541,7 +1813,9 @@ class PcgSolver {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     void *k_init = nullptr, *k_spmv = nullptr, *k_fwd = nullptr, *k_bwd = nullptr, *k_true = nullptr,
          *k_restart = nullptr;
-    void* k_head = nullptr;  // backward head (K = 1)
+    // narrow levels (K = 1): the launch for the factor's value type
+    cudaError_t (*narrow)(SolveArgs&, cudaStream_t) = nullptr;
+    cudaError_t (*narrow_init)() = nullptr;
     void* k_long = nullptr;  // long rows of the SpMV
     // long rows of the one-RHS CSR SpMV (spmv_long_kernel)
     int32_t* lrows = nullptr;
@@ -1551,7 +1825,7 @@ class PcgSolver {
     int32_t *lflag = nullptr, *lpos = nullptr;  // [n], [n + 1]
     void* ltmp = nullptr;                       // scan scratch
 
-    bool use_head() const { return k_head && F.hb_nlev > 0; }
+    bool use_narrow() const { return narrow && F.nf_rows + F.nb_rows > 0; }
 
     // The rows of A longer than kLongRow, ascending: the SpMV gives each its
     // own CTA (the sliced-ELL copy leaves them out).
@@ -1628,14 +1902,7 @@ class PcgSolver {
         a.lrows = lrows;
         a.lr_dot = lr_dot;
         a.n_lrows = n_lrows;
-        if (use_head()) {
-            a.hb_lv = F.hb_lv;
-            a.hb_idx = F.hb_idx;
-            a.hb_nlev = F.hb_nlev;
-            a.hb_ntask = F.hb_ntask;
-            a.hb_rows = F.hb_rows;
-            a.hb_stage = F.hb_stage;
-        }
+        if (use_narrow()) set_narrow(a, F);
         a.b = b;
         a.x = x;
         a.r = r;
@@ -1664,12 +1931,10 @@ class PcgSolver {
         return cudaLaunchKernel(fn, dim3(grid), dim3(kBlock), params, 0, stream);
     }
 
-    // z = L^-T D^+ y: the backward head (one CTA) first, then the rest
+    // z = M^-1 r after launch(k_fwd): the narrow levels, then the rest
     cudaError_t launch_bwd(SolveArgs& a) {
-        if (a.hb_nlev > 0) {
-            void* params[] = {&a};
-            const size_t smem = (size_t)head_smem_bytes(a.hb_rows, a.hb_stage);
-            cudaError_t e = cudaLaunchKernel(k_head, dim3(1), dim3(kHeadThreads), params, smem, stream);
+        if (narrow) {
+            cudaError_t e = narrow(a, stream);
             if (e != cudaSuccess) return e;
         }
         return launch(k_bwd, grid_bwd, a);
@@ -1713,7 +1978,10 @@ static void bind_kernels(PcgSolver* s) {
     s->k_bwd = K == 1 ? (void*)bwd_pack_kernel<TV> : (void*)bwd_kernel<K, TV>;
     s->k_true = (void*)true_residual_kernel<K>;
     s->k_restart = (void*)restart_kernel<K>;
-    s->k_head = K == 1 ? (void*)bwd_head_kernel<TV> : nullptr;
+    if (K == 1) {
+        s->narrow = launch_narrow<TV>;
+        s->narrow_init = narrow_attributes<TV>;
+    }
     s->k_long = K == 1 ? (void*)spmv_long_kernel : (void*)spmv_long_k_kernel<K>;
 }
 
@@ -1765,7 +2033,7 @@ PcgSolver* pcg_create(const DevCsc& A, const DevFactor& F, const SolveConfig& cf
     s->grid_max = std::max(std::max(s->grid_fwd, s->grid_bwd), std::max(s->grid_spmv, s->grid_vec));
     const size_t nv = (size_t)A.n * (size_t)cfg.k;
     cudaError_t e = cudaSuccess;
-    if (s->k_head) e = cudaFuncSetAttribute(s->k_head, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadSmem);
+    if (s->narrow_init) e = s->narrow_init();
     if (e == cudaSuccess) e = cudaMalloc(&s->r, sizeof(double) * std::max<size_t>(nv, 1));
     if (e == cudaSuccess) e = cudaMalloc(&s->p, sizeof(double) * std::max<size_t>(nv, 1));
     if (e == cudaSuccess) e = cudaMalloc(&s->q, sizeof(double) * std::max<size_t>(nv, 1));
@@ -1865,7 +2133,7 @@ cudaError_t pcg_solve(PcgSolver* s, const double* dB, double* dX, SolveResult* r
     if ((e = s->launch(s->k_init, s->grid_vec, a)) != cudaSuccess) return e;
     if ((e = s->launch_start(dB, dX)) != cudaSuccess) return e;
     // per iteration: SpMV, forward, backward (+ the backward head)
-    const int per_it = 3 + (s->use_head() ? 1 : 0) + (s->n_lrows > 0 ? 1 : 0);
+    const int per_it = 3 + (s->use_narrow() ? 1 : 0) + (s->n_lrows > 0 ? 1 : 0);
     res->kernel_launches += per_it;
     if ((e = cudaEventRecord(s->ev1, s->stream)) != cudaSuccess) return e;
     int restarts = 0;
@@ -1956,7 +2224,8 @@ cudaError_t pcg_solve(PcgSolver* s, const double* dB, double* dX, SolveResult* r
 
 // Per-kernel device time of the iteration kernels: starts a solve of dB
 // (tolerance 0, so nothing converges), then times `reps` iterations with an
-// event between every launch.  ms_out[0..2] = mean spmv_update, fwd, bwd.
+// event between every launch.  ms_out[0..2] = mean spmv_update, fwd, bwd (each
+// direction with its narrow levels).
 cudaError_t pcg_profile(PcgSolver* s, const double* dB, double* dX, int reps, float* ms_out) {
     SolveConfig keep = s->cfg;
     s->cfg.tol = 0.0;
@@ -1975,8 +2244,12 @@ cudaError_t pcg_profile(PcgSolver* s, const double* dB, double* dX, int reps, fl
         e = s->launch_spmv(it);
         cudaEventRecord(ev[1], s->stream);
         if (e == cudaSuccess) e = s->launch(s->k_fwd, s->grid_fwd, it);
+        // the narrow levels of each direction in a launch of their own
+        SolveArgs nf = it, nb = it;
+        nf.nb_rows = nf.nb_task = nb.nf_rows = 0;
+        if (e == cudaSuccess && s->narrow) e = s->narrow(nf, s->stream);
         cudaEventRecord(ev[2], s->stream);
-        if (e == cudaSuccess) e = s->launch_bwd(it);
+        if (e == cudaSuccess) e = s->launch_bwd(nb);
         cudaEventRecord(ev[3], s->stream);
         cudaEventSynchronize(ev[3]);
         float m;
@@ -2293,11 +2566,8 @@ class BatchSolver {
     }
     SolveArgs solve_args(const double* b, double* x) {
         SolveArgs a = base->args(b, x);
-        // the batched iteration launches no backward head: every task runs
-        // in the persistent kernel
-        a.hb_lv = nullptr;
-        a.hb_idx = nullptr;
-        a.hb_nlev = a.hb_ntask = a.hb_rows = a.hb_stage = 0;
+        // the batched iteration runs every task in the persistent kernels
+        a.nf_rows = a.nb_rows = a.nb_task = a.hb_nlev = a.hb_ntask = 0;
         a.lrows = nullptr;
         a.lr_dot = nullptr;
         a.n_lrows = 0;
@@ -2597,11 +2867,16 @@ static cudaError_t precond_apply_t(const DevFactor& F, const double* r, double* 
     a.reduce = 0;
     a.timeout_ns = (unsigned long long)(timeout_s * 1e9);
     const int64_t total = (int64_t)F.n * K;
+    if (K == 1) {
+        set_narrow(a, F);
+        e = narrow_attributes<TV>();
+    }
     fill_pending_kernel<<<grid_for(total, kBlock, 8), kBlock, 0, s>>>(y, total);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     const void* kf = K == 1 ? (const void*)fwd_pack_kernel<TV> : (const void*)fwd_kernel<K, TV>;
     const void* kb = K == 1 ? (const void*)bwd_pack_kernel<TV> : (const void*)bwd_kernel<K, TV>;
     if (e == cudaSuccess) e = launch_coresident(kf, resident_blocks(kf, device), a, s);
+    if (e == cudaSuccess && K == 1) e = launch_narrow<TV>(a, s);
     if (e == cudaSuccess) e = launch_coresident(kb, resident_blocks(kb, device), a, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(status, &sc->status, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -2700,11 +2975,16 @@ cudaError_t precond_apply_noalloc_t(const DevFactor& F, const double* r, double*
     a.update = 0;
     a.reduce = 0;
     a.timeout_ns = (unsigned long long)(timeout_s * 1e9);
+    if (K == 1) {
+        set_narrow(a, F);
+        e = narrow_attributes<TV>();
+    }
     fill_pending_kernel<<<grid_for((int64_t)F.n * K, kBlock, 8), kBlock, 0, s>>>(y, (int64_t)F.n * K);
-    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaGetLastError();
     const void* kf = K == 1 ? (const void*)fwd_pack_kernel<TV> : (const void*)fwd_kernel<K, TV>;
     const void* kb = K == 1 ? (const void*)bwd_pack_kernel<TV> : (const void*)bwd_kernel<K, TV>;
     if (e == cudaSuccess) e = launch_coresident(kf, resident_blocks(kf, device), a, s);
+    if (e == cudaSuccess && K == 1) e = launch_narrow<TV>(a, s);
     if (e == cudaSuccess) e = launch_coresident(kb, resident_blocks(kb, device), a, s);
     int st = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&st, &sc->status, sizeof(int), cudaMemcpyDeviceToHost, s);

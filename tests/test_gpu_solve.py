@@ -481,3 +481,45 @@ def test_disconnected_graph_with_isolated_vertex():
         f.free()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("graph", ["strip", "grid2d", "grid27", "power_law", "disconnected"])
+def test_narrow_levels_match_persistent_kernels(graph, fp32):
+    """The narrow levels of both sweeps by the cluster kernel: z is the
+    persistent kernels' bit for bit (bwd_head = 0 switches it off), for a strip
+    whose levels and rows outgrow the cluster's range, a whole system inside
+    it, ranges with many tasks a level, long and split rows, several components
+    and a zero pivot; the allocation-free apply gives the same bits."""
+    torch = pytest.importorskip("torch")
+    if graph == "strip":
+        n, r, c, v, g = grid_laplacian((15000, 2), seed=53, excess_frac=0.05)
+    elif graph == "grid2d":
+        n, r, c, v, g = grid_laplacian((150, 140), seed=51, excess_frac=0.05, wlo=1e-2, whi=1e2)
+    elif graph == "grid27":
+        n, r, c, v, g = R.generate("grid3d27", [17, 16, 18], wlo=0.1, whi=10.0, log_weights=True, aniso_z=100.0,
+                                   excess_frac=1.0, excess_lo=1e-4, excess_hi=1e-4, seed=5)
+    elif graph == "power_law":
+        n, r, c, v, g = R.generate("chunglu", [20000, 150000, 2, 5000], wlo=1.0, whi=10.0, seed=7)
+    else:
+        n, r, c, v = disconnected_laplacian()[:4]
+        g = False
+    zs = []
+    for narrow in (0, 1):
+        ctx = R.Context(seed=6, precision=R.PREC_FP32_FACTOR if fp32 else R.PREC_FP64, bwd_head=narrow)
+        try:
+            ctx.set_triplets(n, r, c, v, trim_ground=g)
+            f = ctx.factor()
+            rr = np.random.default_rng(8).standard_normal(f.info().n)
+            zs.append(ctx.precond_apply(f, rr, fp32=fp32))
+            rd = torch.tensor(rr, device="cuda")
+            zd = torch.empty_like(rd)
+            torch.cuda.synchronize()
+            ctx.precond_apply_noalloc(f, rd.data_ptr(), zd.data_ptr(), 1, fp32, 0)
+            torch.cuda.synchronize()
+            zs.append(zd.cpu().numpy())
+            f.free()
+        finally:
+            ctx.close()
+    for z in zs[1:]:
+        np.testing.assert_array_equal(z, zs[0])
