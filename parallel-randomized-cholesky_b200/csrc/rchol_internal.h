@@ -295,10 +295,11 @@ cudaError_t build_solve_layouts(DevFactor& f, Scratch& sc, cudaStream_t s);
 // up to kNarrowRows rows a direction (each CTA's shared memory holds a copy of
 // their values: 208 of the 227 KB), in levels of at most kNarrowTasks tasks;
 // fewer than kNarrowMinLevels such levels stay with the persistent kernels.
-// 128 tasks: half the cluster's warps.  Solve times with 64 / 128 / 256: 256^2
-// grid 7.0 / 6.3 / 6.3 ms, 61x53x47 (iterations only) 12.8 / 11.4 / 11.4, 128^3
-// one apply 1.02 / 1.01 / 1.10.  16 CTAs against 4 and 1: 256^2 6.3 / 7.0 / 7.7
-// ms (each with the levels that suit it); small systems lose 3% to 4 CTAs.
+// 128 tasks: half the cluster's warps.  Against 256 the 256^2 solve takes 6.26
+// and 6.32 ms, 61x53x47 the same, one 128^3 apply 1.01 and 1.10; 64 was slower than
+// 256 in an earlier form of the kernel (256^2 7.0 against 6.8, 61x53x47 13.2 against
+// 12.4).  16 CTAs against 4 (64 tasks) and 1 (16 tasks): 256^2 6.3 / 7.0 / 7.7 ms;
+// the 2867-vertex grid is 3% faster with 4.
 constexpr int kNarrowCtas = 16;
 constexpr int kNarrowRows = 26 * 1024;
 constexpr int kNarrowTasks = 128;

@@ -1259,18 +1259,18 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) bwd_pack_kernel(Solve
 // slot order and a row's lanes by the shuffle tree of the pack kernels, so y
 // and z equal theirs bit for bit.
 // What bounds it is the latency of one row's chain (see the value, re-read the
-// slots, add, shuffle, store to the other CTAs: about 0.9 us a level down to
-// 0.5 on one CTA, where a store between CTAs alone takes 374 cycles), so the waits
-// and sums are free of data-dependent branches; the persistent kernels spend
-// 1.2 us a level.  Per solve iteration, both sweeps: 2867-vertex grid 114 -> 74
-// us, 256^2 178 -> 137, 61x53x47 530 -> 400, power-law (100k vertices) 3.0 -> 2.5
-// ms; one 128^3 apply (FP32) 1.08 -> 0.99 ms.
+// slots, add, shuffle, store): step stamps gave about 1050 cycles a level with
+// everything on one CTA, and a store seen by another CTA takes 374 cycles more.
+// So the waits and sums are free of data-dependent branches.  Both sweeps of an
+// iteration, each direction profiled in launches of its own: 2867-vertex grid
+// 114 -> 89 us, 256^2 178 -> 152, 61x53x47 530 -> 417, power-law (100k vertices)
+// 3.03 -> 2.52 ms; one 128^3 apply (FP32) 1.08 -> 0.99 ms.
 // With reduce, CTA 0 adds the r.z terms of the first hb_nlev backward levels
 // (see DevFactor::hb_nlev) while the other CTAs solve.
 // ---------------------------------------------------------------------------
 // Form of the kernel: kM slots a lane and chunk, kBufs chunks in flight a
 // warp, values outside the range fetched kLead chunks ahead.  Rows of a few
-// slots want the many warps of NarrowShort (61x53x47 grid, 28 iterations: 11.0
+// slots want the many warps of NarrowShort (61x53x47 grid, 28 iterations: 11.4
 // ms against 12.2 with NarrowLong); rows of many chunks are a serial chain
 // of fetches without NarrowLong's deeper stream (power-law, 100k vertices, 12
 // iterations: 42.4 -> 33.1 ms).
