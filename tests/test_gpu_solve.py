@@ -523,3 +523,32 @@ def test_narrow_levels_match_persistent_kernels(graph, fp32):
             ctx.close()
     for z in zs[1:]:
         np.testing.assert_array_equal(z, zs[0])
+
+
+@pytest.mark.parametrize("m", [2, 33, 34, 258, 259, 700])
+def test_backward_levels_of_long_columns(m):
+    """The backward levels' longest paths for columns of up to m - 1 entries
+    (a complete graph's first column holds all of them): the DAG depth equals
+    the one computed from the factor on the host."""
+    r, c = np.triu_indices(m, 1)
+    w = np.random.default_rng(m).uniform(1.0, 2.0, r.size)
+    deg = np.bincount(r, w, m) + np.bincount(c, w, m)
+    rows = np.concatenate([r, c, np.arange(m)])
+    cols = np.concatenate([c, r, np.arange(m)])
+    vals = np.concatenate([-w, -w, deg])
+    ctx = R.Context(seed=3)
+    try:
+        ctx.set_triplets(m, rows, cols, vals, trim_ground=False)
+        f = ctx.factor()
+        cp, ri, _, _ = f.to_host()
+        depth = f.info().solve_depth_b
+        f.free()
+    finally:
+        ctx.close()
+    lev = np.zeros(m, dtype=np.int64)
+    for j in range(m - 1, -1, -1):
+        below = ri[cp[j]:cp[j + 1]]
+        below = below[below > j]
+        lev[j] = 1 + lev[below].max() if below.size else 0
+    assert int(np.diff(cp).max()) >= m - 1
+    assert depth == lev.max() + 1
