@@ -1895,6 +1895,8 @@ __global__ void count_huge_kernel(const int32_t* __restrict__ colptr, const int3
     }
 }
 
+constexpr int kScatterU = 8;
+
 // Strict lower triangle with |values|, original order within each column
 // (make_lower_triangular, pre_process.hpp:785-867).
 __global__ void scatter_lower_kernel(int32_t n, const int32_t* __restrict__ colptr,
@@ -1934,16 +1936,29 @@ __global__ void scatter_lower_kernel(int32_t n, const int32_t* __restrict__ colp
                 }
                 continue;
             }
-            for (int base = cs; base < ce; base += 32) {
-                const int p = base + lane;
-                const bool take = p < ce && rowind[p] > cc;
-                const unsigned bal = __ballot_sync(kFull, take);
-                if (take) {
-                    const int at = out + __popc(bal & ((1u << lane) - 1u));
-                    lrow[at] = rowind[p];
-                    lval[at] = fabs(val[p]);
+            // kScatterU chunks' loads in flight: chunk by chunk a hub's column is one
+            // memory round trip after the other (power-law, 100k vertices: 1.08
+            // -> 0.23 ms)
+            for (int base = cs; base < ce; base += 32 * kScatterU) {
+                int32_t r[kScatterU];
+                double v[kScatterU];
+#pragma unroll
+                for (int u = 0; u < kScatterU; ++u) {
+                    const int p = base + 32 * u + lane;
+                    r[u] = p < ce ? rowind[p] : -1;
+                    v[u] = p < ce ? val[p] : 0.0;
                 }
-                out += __popc(bal);
+#pragma unroll
+                for (int u = 0; u < kScatterU; ++u) {
+                    const bool take = r[u] > cc;
+                    const unsigned bal = __ballot_sync(kFull, take);
+                    if (take) {
+                        const int at = out + __popc(bal & ((1u << lane) - 1u));
+                        lrow[at] = r[u];
+                        lval[at] = fabs(v[u]);
+                    }
+                    out += __popc(bal);
+                }
             }
         }
     }

@@ -328,6 +328,28 @@ def test_cta_elimination_list_sizes(N, tail):
     assert info.max_gather >= N
 
 
+@pytest.mark.parametrize("length", [64, 255, 256, 257, 511, 513, 1100])
+def test_lower_triangle_of_long_columns(length):
+    """A hub in the middle of the order, its column `length` entries long and
+    about half of them below the diagonal: the set-up takes them eight
+    32-entry chunks at a time, in order: bit-exact."""
+    rng = np.random.default_rng(length)
+    hub = length // 2
+    n = length  # the column holds the diagonal too
+    other = np.array([i for i in range(n) if i != hub])
+    a = np.concatenate([np.full(n - 1, hub), np.arange(n - 1)])
+    b = np.concatenate([other, np.arange(1, n)])
+    keep = (a != hub) & (b != hub) | (np.arange(len(a)) < n - 1)
+    a, b = a[keep], b[keep]
+    w = rng.uniform(0.5, 2.0, len(a))
+    d = np.bincount(a, weights=w, minlength=n) + np.bincount(b, weights=w, minlength=n)
+    i = np.arange(n)
+    r, c, v = np.concatenate([a, b, i]), np.concatenate([b, a, i]), np.concatenate([-w, -w, d])
+    orc = OracleProblem(n, r, c, v).factor(seed=5)
+    gpu, _ = _gpu_factor(n, r, c, v, False, 5)
+    _compare(gpu, orc)
+
+
 def test_autotune_choices_are_used_and_cached():
     """rchol_autotune profiles the gathers, keeps only choices that time
     faster, writes them into the context's options (the next factorization
