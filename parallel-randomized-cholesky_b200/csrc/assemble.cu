@@ -992,7 +992,7 @@ static cudaError_t build_narrow(DevFactor& f, const int32_t* levf, const int32_t
     clear_narrow(f);
     const int32_t cf = std::min<int32_t>(f.depth, kNarrowMaxLevels), lf0 = f.depth - cf;
     const int32_t cb = std::min<int32_t>(f.depth_b, kNarrowMaxLevels);
-    if (f.npt_b == 0 || std::max(cf, cb) < kNarrowMinLevels) return cudaSuccess;
+    if (f.npt_b == 0 || std::max(cf, cb) < kNarrowMinLevels || !narrow_fits()) return cudaSuccess;
     // both level tables behind two flag words, brought over in one copy
     int4* lv = nullptr;
     const int64_t nlv = (int64_t)cf + cb + 3;

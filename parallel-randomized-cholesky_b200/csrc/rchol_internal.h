@@ -305,6 +305,7 @@ constexpr int kNarrowRows = 26 * 1024;
 constexpr int kNarrowTasks = 128;
 constexpr int kNarrowMinLevels = 8;
 constexpr int kNarrowMaxLevels = 16384;
+bool narrow_fits();  // the current device holds such a cluster
 
 // The rows whose r.z terms are summed apart (DevFactor::hb_nlev): the
 // backward levels from the first while each holds at most kHeadMaxRows rows,

@@ -1790,6 +1790,32 @@ int resident_blocks(const void* fn, int device) {
 
 }  // namespace
 
+// Whether the device runs a whole cluster of narrow_kernel's with the largest
+// range at once (a partition of a GPU may hold too few SMs side by side).
+bool narrow_fits() {
+    if (narrow_attributes<double>() != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kNarrowCtas);
+    cfg.blockDim = dim3(NarrowShort::kThreads);
+    cfg.dynamicSmemBytes = sizeof(double) * kNarrowRows;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kNarrowCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)narrow_kernel<double, NarrowShort>, &cfg) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
+}
+
 // ===========================================================================
 
 class PcgSolver {
