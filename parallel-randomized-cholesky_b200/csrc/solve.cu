@@ -1038,10 +1038,12 @@ __device__ __forceinline__ double pack_dot(const PackLane<TV>& L, int lane, int 
     return sum;
 }
 
-// Sum over the G lanes of each row group (all 32 lanes take part).
+// Sum over the G lanes of each row group (all 32 lanes take part).  A plain
+// loop over the group's own steps: it is on every row's critical path.  Unrolled
+// to 16..1 with a test each, one 128^3 apply takes 993 us, not 962 (a switch
+// into the steps: 985), and the 128^3 solve 31.3 ms, not 30.2.
 __device__ __forceinline__ double group_sum(double v, int G) {
-    for (int o = 16; o > 0; o >>= 1)
-        if (o < G) v += __shfl_xor_sync(kFull, v, o);
+    for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     return v;
 }
 
@@ -1261,10 +1263,11 @@ __global__ void __launch_bounds__(kBlock, RCHOL_PACK_MINB) bwd_pack_kernel(Solve
 // What bounds it is the latency of one row's chain (see the value, re-read the
 // slots, add, shuffle, store): step stamps gave about 1050 cycles a level with
 // everything on one CTA, and a store seen by another CTA takes 374 cycles more.
-// So the waits and sums are free of data-dependent branches.  Both sweeps of an
+// So the waits are free of data-dependent branches, and the sums take no step
+// beyond the row's own.  Both sweeps of an
 // iteration, each direction profiled in launches of its own: 2867-vertex grid
-// 114 -> 89 us, 256^2 178 -> 152, 61x53x47 530 -> 417, power-law (100k vertices)
-// 3.03 -> 2.52 ms; one 128^3 apply (FP32) 1.08 -> 0.99 ms.
+// 114 -> 89 us, 256^2 178 -> 144, 61x53x47 530 -> 394, power-law (100k vertices)
+// 3.03 -> 2.52 ms; one 128^3 apply (FP32) 1.08 -> 0.95 ms.
 // With reduce, CTA 0 adds the r.z terms of the first hb_nlev backward levels
 // (see DevFactor::hb_nlev) while the other CTAs solve.
 // ---------------------------------------------------------------------------
@@ -1404,7 +1407,7 @@ __device__ bool narrow_tasks(const SolveArgs& a, double* copy, int id, int nw, i
             if (!FWD && c.dj != 0.0) tj = tj / c.dj;
             asm volatile("" : "+d"(tj));  // the division stays ahead of the waits
             if (c.k0 == 0) sum = 0.0;
-            // Waits and sums hold no data-dependent branch: from the last
+            // The waits hold no data-dependent branch: from the last
             // dependency's arrival to the store every instruction counts.
             // The row's gate (its last dependency) alone first, then all slots.
             unsigned spins = 0;
@@ -1440,14 +1443,7 @@ __device__ bool narrow_tasks(const SolveArgs& a, double* copy, int id, int nw, i
                 for (int k = 4; k < kM; ++k) sum += to_d(c.val[k]) * (c.idx[k] >= 0 ? v[k] : c.out[k]);
             }
             if (c.k0 + kM >= m) {
-                switch (cls) {
-                    case 5: sum += __shfl_xor_sync(kFull, sum, 16); [[fallthrough]];
-                    case 4: sum += __shfl_xor_sync(kFull, sum, 8); [[fallthrough]];
-                    case 3: sum += __shfl_xor_sync(kFull, sum, 4); [[fallthrough]];
-                    case 2: sum += __shfl_xor_sync(kFull, sum, 2); [[fallthrough]];
-                    case 1: sum += __shfl_xor_sync(kFull, sum, 1); [[fallthrough]];
-                    default: break;
-                }
+                sum = group_sum(sum, G);
                 const bool in = (lane >> cls) < cnt;
                 double* at = copy + (c.pos - p0) + (lane >> cls);
                 if (!((c.dz >> 11) & 1)) {
