@@ -426,7 +426,10 @@ __device__ __forceinline__ bool pool_take(const FactorArgs& a, int m, int lane, 
 }
 
 // The release of the cooperative passes: no queue, a CTA waits on the counter
-// itself.  The caller's fence orders the column's writes before it.
+// itself.  The column's fills, levels and counter increments come from all
+// threads of the warp or CTA: a barrier first, then the releasing thread's own
+// __threadfence, then this.  (A fence that each thread passes before the barrier
+// orders only its own writes before its own atomics, not the other threads'.)
 __device__ __forceinline__ void release_row(const FactorArgs& a, int32_t r, int mult) { atomicAdd(a.dep + r, -mult); }
 
 // Elimination of a vertex whose gathered list fits one warp (at most 32
@@ -565,13 +568,17 @@ __device__ bool eliminate_small(const FactorArgs& a, int32_t k, int total, int32
         return false;
     }
     const int lk = lvl + 1;
-    if (!QUEUE && lane < m) atomicMax(a.level + mrow, lk);
-    __threadfence();
-    __syncwarp();
     if (QUEUE) {
+        __threadfence();
+        __syncwarp();
         release_chunk(a, lk, lane, lane < m, mrow, mcnt, next);
-    } else if (lane < m) {
-        release_row(a, mrow, mcnt);
+    } else {
+        if (lane < m) atomicMax(a.level + mrow, lk);
+        __syncwarp();
+        if (lane < m) {
+            __threadfence();
+            release_row(a, mrow, mcnt);
+        }
     }
     __syncwarp();
     return true;
@@ -1466,11 +1473,11 @@ __device__ __forceinline__ bool cta_eliminate(const FactorArgs& a, const CtaVert
     }
     // fills, pool writes and levels are visible before any neighbour is
     // released: each neighbour's counter drops by its multiplicity
-    __threadfence();
     if (__syncthreads_or(!ok)) {
         if (tid == 0) fail(a, kDevCapacity);
         return false;
     }
+    if (tid < m) __threadfence();
     for (int i = tid; i < m; i += NT) release_row(a, orow[i], mult[i]);
     fills += m - 1;
     return true;
@@ -1738,11 +1745,11 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 1) factor_cta_kernel(Facto
                 if (!append_fill(a, ri > rj ? rj : ri, grow, __ddiv_rn(__dmul_rn(s.b_val[i], rem_i), S))) ok = false;
                 atomicAdd(a.dep + grow, 1);
             }
-            __threadfence();
             if (__syncthreads_or(!ok)) {
                 if (tid == 0) fail(a, kDevCapacity);
                 break;
             }
+            if (tid < m) __threadfence();
             for (int i = tid; i < m; i += NT) release_row(a, s.b_row[i], (int)(s.b_aux[i] >> 32));
             fills += m - 1;
             if (lock >= 0) {
