@@ -992,9 +992,16 @@ __global__ void __launch_bounds__(256, 3) factor_kernel(FactorArgs a) {
 // SM, for the hubs and the dense core of power-law graphs (the tail_vertices
 // option).
 
-// Sorts n keys (tag, value bits), thread t holding positions t, t + NT, ...
-// (positions past n hold the greatest key): by (tag, value bits), or, BYVAL, by
-// value bits with ties in entry order (the tag must be the position on entry).
+// A value's bits as a sort key.  Nonnegative values order as their bits and a
+// NaN, of either sign, comes after them; the keys of the padding, all ones, must
+// come after that, and cta_sort adds one to a key, so the NaN of all ones gives up
+// its last bit.
+constexpr unsigned long long kPadKey = ~0ull;
+__device__ __forceinline__ unsigned long long key_bits(unsigned long long v) { return v < kPadKey ? v : kPadKey - 1; }
+
+// Sorts n keys (tag, value bits below kPadKey), thread t holding positions t,
+// t + NT, ... (positions past n hold the greatest key): by (tag, value bits), or,
+// BYVAL, by value bits with ties in entry order (the tag must be the position on entry).
 // The sorted keys end in the registers by position and in one of the buffer
 // pairs (x0, r0), (x1, r1), which is returned (0 or 1).  Ends with a barrier.
 // The comparisons are written without short circuits: as branches they took
@@ -1300,7 +1307,7 @@ __device__ __forceinline__ bool cta_eliminate(const FactorArgs& a, const CtaVert
                 tg[e] = a.lrow[V.o0 + i - V.n0];
                 v = a.lval[V.o0 + i - V.n0];
             }
-            vb[e] = i < total ? (unsigned long long)__double_as_longlong(v) : ~0ull >> 1;
+            vb[e] = i < total ? key_bits((unsigned long long)__double_as_longlong(v)) : kPadKey;
         }
     } else {
         double* g = reinterpret_cast<double*>(x1);
@@ -1333,7 +1340,7 @@ __device__ __forceinline__ bool cta_eliminate(const FactorArgs& a, const CtaVert
         for (int e = 0; e < EE; ++e) {
             const int i = e * NT + tid;
             tg[e] = i < total ? r1[i] : INT_MAX;
-            vb[e] = i < total ? x1[i] : ~0ull >> 1;
+            vb[e] = i < total ? key_bits(x1[i]) : kPadKey;
         }
     }
     // ---- sort by (row, value bits); merge duplicate rows in that order
@@ -1400,7 +1407,7 @@ __device__ __forceinline__ bool cta_eliminate(const FactorArgs& a, const CtaVert
     for (int e = 0; e < EE; ++e) {
         const int i = e * NT + tid;
         tg[e] = i;
-        vb[e] = i < m ? ox[i] : ~0ull >> 1;
+        vb[e] = i < m ? key_bits(ox[i]) : kPadKey;
     }
     const int c2 = cta_sort<NT, EE, true>(tg, vb, m, fx, ox, fr, r2);
     double* C = reinterpret_cast<double*>(c2 ? fx : ox);  // the buffers the sort left free
