@@ -103,20 +103,23 @@ __device__ void sort_row_value(int32_t* row, double* val, int P, int lane) {
     }
 }
 
-// ascending by (value, row) carrying aux
+// ascending by (value bits, row) carrying aux.  Nonnegative values order as their
+// bits; compared as doubles, a NaN would leave the network in no order at all and
+// let padding (all ones, row INT_MAX) in before entries of the list.
 __device__ void sort_value_row(double* val, int32_t* row, long long* aux, int P, int lane) {
     for (int k = 2; k <= P; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
             for (int i = lane; i < P; i += kWarp) {
                 int l = i ^ j;
                 if (l > i) {
-                    double vi = val[i], vl = val[l];
                     int32_t ri = row[i], rl = row[l];
+                    unsigned long long vi = (unsigned long long)__double_as_longlong(val[i]);
+                    unsigned long long vl = (unsigned long long)__double_as_longlong(val[l]);
                     bool gt = (vi > vl) | ((vi == vl) & (ri > rl));
                     bool asc = (i & k) == 0;
                     if (gt == asc) {
-                        val[i] = vl;
-                        val[l] = vi;
+                        val[i] = __longlong_as_double((long long)vl);
+                        val[l] = __longlong_as_double((long long)vi);
                         row[i] = rl;
                         row[l] = ri;
                         long long ai = aux[i];
@@ -781,7 +784,7 @@ __device__ __forceinline__ bool eliminate_slab(const FactorArgs& a, int32_t k, i
     const int P2 = pow2_at_least(m);
     if (!global) {
         for (int t = m + lane; t < P2; t += kWarp) {
-            s.b_val[t] = __longlong_as_double((long long)kInfBits);
+            s.b_val[t] = __longlong_as_double(-1ll);
             s.b_row[t] = INT_MAX;
             s.b_aux[t] = 0;
         }

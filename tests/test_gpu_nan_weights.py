@@ -76,3 +76,8 @@ def test_late_vertices_of_a_256_thread_cta(N):
 @pytest.mark.parametrize("N", [40, 1000, 1500, 3000, 4094])
 def test_late_vertices_of_a_1024_thread_cta(N):
     check(N, before=8, after=0, tail_vertices=N + 2)
+
+
+@pytest.mark.parametrize("N", [20, 33, 40, 100, 128, 200, 255, 300, 1000])
+def test_early_vertices_of_one_warp(N):
+    check(N, before=0, after=8 * (N + 40))
