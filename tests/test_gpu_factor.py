@@ -328,6 +328,17 @@ def test_cta_elimination_list_sizes(N, tail):
     assert info.max_gather >= N
 
 
+@pytest.mark.parametrize("n,edges", [(30000, 300000), (50000, 500000)])
+def test_first_factorization_of_long_lists(n, edges):
+    """A power-law graph with short columns below the diagonal but lists of
+    1024 to 4096 entries at its late vertices: factored at the first attempt."""
+    n, r, c, v, g = R.generate("chunglu", [n, edges, 2, n // 4], wlo=1.0, whi=10.0, seed=7)
+    lower = np.bincount(np.minimum(r, c)[np.asarray(r) > np.asarray(c)], minlength=n)
+    _, info = _gpu_factor(n, r, c, v, g, 4)
+    assert lower.max() <= 256 and 1024 < info.max_gather <= 4096
+    assert info.attempts == 1
+
+
 @pytest.mark.parametrize("length", [64, 255, 256, 257, 511, 513, 1100])
 def test_lower_triangle_of_long_columns(length):
     """A hub in the middle of the order, its column `length` entries long and
