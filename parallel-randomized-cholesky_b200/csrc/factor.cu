@@ -12,7 +12,7 @@
 //     slot), so the factor does not depend on which warp took which vertex;
 //   * fill edges are appended to per-column buckets by atomics (driver.cu
 //     used an open-addressing hash over 4*nnz slots, :1068-1150): a fixed
-//     first chunk per column plus 64-entry overflow chunks linked lock-free.
+//     first chunk per column plus linked overflow chunks.
 // FP64 arithmetic uses explicitly rounded intrinsics (no contraction), which
 // makes the factor bit-identical to the CPU oracle's ORC_MODE_B200.
 #include <algorithm>
@@ -341,14 +341,24 @@ __device__ __forceinline__ void fail(const FactorArgs& a, int code) {
     atomicExch(a.counters + kAbort, 1);
 }
 
-// Append one fill edge (row > col) to column col's bucket.  Returns false on
-// pool exhaustion.  Chunks are linked with CAS, so no thread ever waits.
+// Append one fill edge (row > col) to column col's bucket.  Returns false when
+// the kernel must stop.
 __device__ bool store_fill(const FactorArgs& a, int32_t col, int32_t row, double v, int s);
 __device__ __forceinline__ bool append_fill(const FactorArgs& a, int32_t col, int32_t row, double v) {
     return store_fill(a, col, row, v, atomicAdd(a.fcnt + col, 1));
 }
 
 // Fill number s of column col (reserved by the atomic add on its count).
+// Overflow chunk number ci of a column spans kChunk << ci slots (2^ci pool
+// units), so slot t is at most log2(t / kChunk + 1) links away.  The thread that
+// holds a chunk's first slot claims its units and links it; the others wait for
+// the link.  (When every thread that met an empty link claimed units and the
+// losers of the link kept theirs, a 100k-vertex power-law graph took 65.6k units,
+// by the run a little more or less, where its columns call for 37.7k of the pool's
+// 72.9k; a pool that runs out costs a whole second attempt.)
+// A wait ends: the claiming thread reserved its slot earlier and is on its
+// way here, itself waiting at most for earlier chunks of the column, and every
+// round of the loop serves all lanes of the warp.
 __device__ bool store_fill(const FactorArgs& a, int32_t col, int32_t row, double v, int s) {
     if (s < a.c0) {
         size_t o = (size_t)col * (size_t)a.c0 + (size_t)s;
@@ -357,29 +367,44 @@ __device__ bool store_fill(const FactorArgs& a, int32_t col, int32_t row, double
         return true;
     }
     atomicAdd(a.counters + kOverflowFills, 1);
-    // overflow chunk number lvl of a column spans kChunk << lvl slots (2^lvl
-    // pool units), so slot t is at most log2(t / kChunk + 1) links away
     const int t = s - a.c0;
     const int ci = 31 - __clz(t / kChunk + 1);
     const int off = t - kChunk * ((1 << ci) - 1);
     int32_t* link = a.chead + col;
-    int cur = -1;
-    for (int lvl = 0;; ++lvl) {
-        cur = ld_relaxed(link);
-        if (cur < 0) {
-            const int units = 1 << lvl;
+    int lvl = 0;
+    unsigned spins = 0;
+    unsigned long long since = 0;
+    while (true) {
+        int cur = ld_relaxed(link);
+        if (cur < 0 && lvl == ci && off == 0) {
+            const int units = 1 << ci;
             const int nc = atomicAdd(a.counters + kChunkCursor, units);
-            if (nc > a.nchunks - units) return false;
-            const int old = atomicCAS(link, -1, nc);
-            cur = (old == -1) ? nc : old;
+            if (nc > a.nchunks - units) {
+                fail(a, kDevCapacity);
+                return false;
+            }
+            atomicExch(link, nc);
+            cur = nc;
         }
-        if (lvl == ci) break;
-        link = a.cnext + cur;
+        if (cur >= 0) {
+            if (lvl == ci) {
+                size_t o = (size_t)cur * kChunk + (size_t)off;
+                a.crow[o] = row;
+                a.cval[o] = v;
+                return true;
+            }
+            link = a.cnext + cur;
+            ++lvl;
+        } else if ((++spins & 63u) == 0) {
+            if (aborted(a)) return false;
+            const unsigned long long now = global_timer_ns();
+            if (since == 0) since = now;
+            if (now - since > a.timeout_ns) {
+                fail(a, kDevTimeout);
+                return false;
+            }
+        }
     }
-    size_t o = (size_t)cur * kChunk + (size_t)off;
-    a.crow[o] = row;
-    a.cval[o] = v;
-    return true;
 }
 
 // Release one chunk of merged neighbours after the elimination of a column:

@@ -339,6 +339,25 @@ def test_first_factorization_of_long_lists(n, edges):
     assert info.attempts == 1
 
 
+@pytest.mark.parametrize("n,edges,tail", [(6000, 30000, 0), (30000, 300000, 0), (30000, 300000, 700),
+                                          (100000, 1000000, 1500)])
+def test_overflow_chunks_claimed_once(n, edges, tail):
+    """The first factorization of a power-law graph: each overflow chunk of a
+    column is claimed once, however many threads of the grid append to it, so
+    the units used are those that the columns' fill counts call for (the
+    oracle's: 64 slots in the column itself, then chunks of 64, 128, ... in
+    units of 64) and the pool that the context sets up suffices."""
+    n, r, c, v, g = R.generate("chunglu", [n, edges, 2, n // 4], wlo=1.0, whi=10.0, seed=7)
+    P = OracleProblem(n, r, c, v, trim=g)
+    lower = np.bincount(np.minimum(r, c)[np.asarray(r) > np.asarray(c)], minlength=n)
+    over = np.minimum(lower, 64) + P.factor(seed=4)["fills_received"] - 64
+    levels = np.floor(np.log2(np.maximum(over - 1, 0) // 64 + 1)).astype(int) + 1
+    units = np.where(over > 0, 2 ** levels - 1, 0).sum()
+    _, info = _gpu_factor(n, r, c, v, g, 4, tail_vertices=tail)
+    assert info.attempts == 1
+    assert info.chunks_used == units and units > 0
+
+
 @pytest.mark.parametrize("length", [64, 255, 256, 257, 511, 513, 1100])
 def test_lower_triangle_of_long_columns(length):
     """A hub in the middle of the order, its column `length` entries long and
