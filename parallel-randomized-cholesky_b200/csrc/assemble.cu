@@ -703,6 +703,7 @@ cudaError_t assemble_factor(const FactorWork& w, bool trim_ground, bool make_fp3
     if (make_fp32) RCHOL_TRY(realloc_if(&f.diag32, grow_n, capn));
     f.cap_n = capn;
     col_counts_kernel<<<grid_for(nout, 256), 256, 0, s>>>(nout, ground, w.pcnt, w.pstart, w.prow, cnt);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(exclusive_scan_i32_to_i64(cnt, f.lc_ptr, nout, tmp, s));
     int64_t nnz = 0;
@@ -739,16 +740,19 @@ cudaError_t assemble_factor(const FactorWork& w, bool trim_ground, bool make_fp3
     RCHOL_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(nout > 0 ? nout : 1), s));
     scatter_cols_kernel<<<grid_for((int64_t)nout * 32, 256), 256, 0, s>>>(nout, f.lc_ptr, w.pstart, w.prow, w.pval,
                                                                           f.lc_idx, f.lc_val, cnt, col_of);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(exclusive_scan_i32_to_i64(cnt, f.lr_ptr, nout, tmp, s));
     if (by_sort) {
         RCHOL_TRY(stable_key_order_carried(f.lc_idx, (int32_t)nnz, nout, eorder, sc, s));
         gather_rows_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(nnz, eorder, col_of, f.lc_val, f.lr_idx, f.lr_val);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     } else {
         RCHOL_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(nout > 0 ? nout : 1), s));
         transpose_kernel<<<grid_for((int64_t)nout * 32, 256), 256, 0, s>>>(nout, f.lc_ptr, f.lc_idx, f.lc_val,
                                                                            f.lr_ptr, cnt, f.lr_idx, f.lr_val);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     // deterministic row order: warp sort for short rows, CTA sort for long ones
@@ -756,9 +760,12 @@ cudaError_t assemble_factor(const FactorWork& w, bool trim_ground, bool make_fp3
     const int sort_grid = current_sm_count() * 4;
     RCHOL_TRY(cudaMemsetAsync(dsc, 0, sizeof(int32_t) * 4, s));  // long rows, max row, max level
     max_kernel<<<grid_for(nout, 256), 256, 0, s>>>(cnt, nout, dsc + 1);
+    count_launch();
     max_kernel<<<grid_for(nout, 256), 256, 0, s>>>(w.level, nout, dsc + 2);
+    count_launch();
     if (!by_sort) {
         sort_rows_kernel<<<sort_grid, sort_block, 0, s>>>(nout, f.lr_ptr, f.lr_idx, f.lr_val, long_rows, dsc);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     int32_t hs[4] = {0, 0, 0, 0};
@@ -778,6 +785,7 @@ cudaError_t assemble_factor(const FactorWork& w, bool trim_ground, bool make_fp3
         RCHOL_TRY(cudaFuncSetAttribute(sort_long_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         sort_long_rows_kernel<<<lgrid, 512, smem, s>>>(long_rows, hs[0], f.lr_ptr, f.lr_idx, f.lr_val, gkey, gval,
                                                         gcap, w.counters + 3);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     f.depth = hs[2] + 1;
@@ -785,8 +793,11 @@ cudaError_t assemble_factor(const FactorWork& w, bool trim_ground, bool make_fp3
     RCHOL_TRY(cudaMemcpyAsync(f.diag, w.diag, sizeof(double) * (size_t)nout, cudaMemcpyDeviceToDevice, s));
     if (make_fp32) {
         to_f32_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(f.lc_val, f.lc_val32, nnz);
+        count_launch();
         to_f32_kernel<<<grid_for(nnz, 256), 256, 0, s>>>(f.lr_val, f.lr_val32, nnz);
+        count_launch();
         to_f32_kernel<<<grid_for(nout, 256), 256, 0, s>>>(f.diag, f.diag32, nout);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     RCHOL_TRY(build_solve_schedule(f, w.level, epl, exact_bwd, bwd_head, timeout_s, sc, s));
@@ -816,9 +827,11 @@ static cudaError_t build_one_schedule(const int32_t* level, const int64_t* ptr, 
         const int grid = nsh > 0 ? grid_for(n, 256, 4) : grid_for(n, 256);
         sched_hist_kernel<<<grid, 256, sizeof(int32_t) * (size_t)nsh, s>>>(level, ptr, n, depth, backward, epl,
                                                                            key, hist, nsh);
+        count_launch();
     }
     RCHOL_TRY(exclusive_scan_i32_to_i32(hist, start, nb, tmp, s));
     sched_task_count_kernel<<<grid_for(nb, 256), 256, 0, s>>>(hist, nb, tcount);
+    count_launch();
     RCHOL_TRY(exclusive_scan_i32_to_i32(tcount, tstart, nb, tmp, s));
     int32_t nt = 0;
     RCHOL_TRY(cudaMemcpyAsync(&nt, tstart + nb, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -826,6 +839,7 @@ static cudaError_t build_one_schedule(const int32_t* level, const int64_t* ptr, 
     *ntasks = nt;
     RCHOL_TRY(ensure(tasks, tcap, (int64_t)nt));
     sched_task_emit_kernel<<<grid_for(nt, 256), 256, 0, s>>>(hist, start, tstart, nb, nt, *tasks);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     return stable_key_order(key, n, nb, order, sc, s);
 }
@@ -838,9 +852,11 @@ static cudaError_t build_layout(int32_t n, const int32_t* order, const int64_t* 
     RCHOL_TRY(sc.get(&len, n));
     RCHOL_TRY(sc.get((char**)&tmp, (int64_t)scan_tmp_bytes(n)));
     permute_len_kernel<<<grid_for(n, 256), 256, 0, s>>>(n, order, ptr, len);
+    count_launch();
     RCHOL_TRY(exclusive_scan_i32_to_i64(len, optr, n, tmp, s));
     permute_rows_kernel<<<grid_for((int64_t)n * 32, 256), 256, 0, s>>>(n, order, ptr, idx, val, val32, optr, oidx,
                                                                         oval, oval32);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -891,6 +907,7 @@ static cudaError_t build_pack(int32_t ntasks, const int2* tasks, const int32_t* 
     }
     pack_nsub_kernel<<<grid_for(ntasks, 256), 256, 0, s>>>(tasks, ntasks, order, ptr, split_min, split_len, nsub,
                                                            issplit);
+    count_launch();
     RCHOL_TRY(exclusive_scan_i32_to_i32(nsub, tbase, ntasks, tmp, s));
     RCHOL_TRY(exclusive_scan_i32_to_i32(issplit, sid, ntasks, tmp, s));
     int32_t hs[2] = {0, 0};
@@ -904,6 +921,7 @@ static cudaError_t build_pack(int32_t ntasks, const int2* tasks, const int32_t* 
         int32_t* psub = nullptr;
         RCHOL_TRY(sc.get(&psub, nt));
         mask_mul_kernel<<<grid_for(ntasks, 256), 256, 0, s>>>(nsub, issplit, psub, ntasks);
+        count_launch();
         RCHOL_TRY(exclusive_scan_i32_to_i32(psub, pbase, ntasks, tmp, s));
         RCHOL_TRY(cudaMemcpyAsync(&nparts, pbase + ntasks, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         RCHOL_TRY(cudaStreamSynchronize(s));
@@ -924,7 +942,9 @@ static cudaError_t build_pack(int32_t ntasks, const int2* tasks, const int32_t* 
     RCHOL_TRY(cudaMemsetAsync(*o.pcount, 0, sizeof(int32_t) * (size_t)std::max<int32_t>(nsp, 1), s));
     pack_expand_kernel<<<grid_for(ntasks, 256), 256, 0, s>>>(tasks, ntasks, ptr, order, split_len, nsub, tbase, sid,
                                                              pbase, etask, *o.split, *o.srow);
+    count_launch();
     pack_m_kernel<<<grid_for(ne, 256), 256, 0, s>>>(etask, ne, order, ptr, m);
+    count_launch();
     RCHOL_TRY(exclusive_scan_i32_to_i64(m, base, ne, tmp2, s));
     int64_t units = 0;
     RCHOL_TRY(cudaMemcpyAsync(&units, base + ne, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -944,9 +964,11 @@ static cudaError_t build_pack(int32_t ntasks, const int2* tasks, const int32_t* 
         *o.cap_w = 0;
     }
     pack_desc_kernel<<<grid_for(ne, 256), 256, 0, s>>>(etask, ne, m, base, *o.pack);
+    count_launch();
     pack_fill_kernel<<<grid_for((int64_t)ne * 32, 256), 256, 0, s>>>(
         *o.pack, ne, order, ptr, split_len, sidx, sval, sval32, level, sign, *o.pidx, *o.pval,
         sval32 ? *o.pval32 : nullptr);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -971,6 +993,7 @@ static cudaError_t build_packs(DevFactor& f, const int32_t* level_f, const int32
     (void)level_f;
     *pos_out = pos_f;
     invert_order_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(f.n, f.order_f, pos_f);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(build_pack(f.ntasks_f, f.tasks_f, f.order_f, f.lr_ptr, f.lr_idx, f.lr_val, f.lr_val32, pos_f, 1,
                          kSplitMinF, kSplitLenF, of, sc, s));
@@ -1002,8 +1025,10 @@ static cudaError_t build_narrow(DevFactor& f, const int32_t* levf, const int32_t
     RCHOL_TRY(cudaMemsetAsync(flags, 0x7f, sizeof(int4), s));
     level_table_kernel<<<grid_for(f.npt_f, 256), 256, 0, s>>>(f.npt_f, f.pack_f, f.order_f, levf, f.n, lf0, cf, lvf,
                                                               flags);
+    count_launch();
     level_table_kernel<<<grid_for(f.npt_b, 256), 256, 0, s>>>(f.npt_b, f.pack_b, f.order_b, levb, f.n, 0, cb, lvb,
                                                               flags + 1);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     std::vector<int4> h((size_t)nlv);
     RCHOL_TRY(cudaMemcpyAsync(h.data(), lv, sizeof(int4) * h.size(), cudaMemcpyDeviceToHost, s));
@@ -1033,6 +1058,7 @@ static cudaError_t build_narrow(DevFactor& f, const int32_t* levf, const int32_t
         f.nf_rows = hf[cf].z - hf[nf].z;
         narrow_idx_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(nslots, f.pf_idx + (int64_t)f.nf_unit * 32, pos_f,
                                                                 f.nf_pos, f.nf_rows, f.nf_idx);
+        count_launch();
     }
     if (nb >= kNarrowMinLevels) {
         const int64_t nslots = (int64_t)hb[nb].y * 32;
@@ -1042,7 +1068,9 @@ static cudaError_t build_narrow(DevFactor& f, const int32_t* levf, const int32_t
         f.nb_task = hb[nb].x;
         f.nb_rows = hb[nb].z;
         invert_order_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(f.n, f.order_b, pos);
+        count_launch();
         narrow_idx_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(nslots, f.pb_idx, pos, 0, f.nb_rows, f.nb_idx);
+        count_launch();
     }
     // slots per lane of the mean narrow task: stencil factors 2.6 to 4.3, a power-law one 6.6
     const int64_t units = (f.nf_rows ? hf[cf].y - hf[nf].y : 0) + (f.nb_rows ? hb[nb].y : 0);
@@ -1129,8 +1157,10 @@ cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bo
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bwd_level_kernel, 256, 0);
     bwd_level_kernel<<<std::max(1, per_sm * sms), 256, 0, s>>>(f.n, f.lc_ptr, f.lc_idx, f.order_f, levb, st,
                                                               (unsigned long long)(timeout_s * 1e9));
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     max_kernel<<<grid_for(f.n, 256), 256, 0, s>>>(levb, f.n, st + 1);
+    count_launch();
     int32_t hs[2] = {0, 0};
     RCHOL_TRY(cudaMemcpyAsync(hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s));
     RCHOL_TRY(cudaStreamSynchronize(s));
@@ -1146,12 +1176,14 @@ cudaError_t build_solve_schedule(DevFactor& f, const int32_t* level, int epl, bo
 
 cudaError_t max_i32(const int32_t* v, int64_t n, int32_t* out, cudaStream_t s) {
     max_kernel<<<grid_for(n, 256), 256, 0, s>>>(v, n, out);
+    count_launch();
     return cudaGetLastError();
 }
 
 cudaError_t check_colptr(const int32_t* colptr, int32_t n, int32_t nnz, int32_t* flag, cudaStream_t s) {
     RCHOL_TRY(cudaMemsetAsync(flag, 0, sizeof(int32_t), s));
     colptr_check_kernel<<<grid_for((int64_t)n + 1, 256), 256, 0, s>>>(colptr, n, nnz, flag);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -1180,12 +1212,14 @@ cudaError_t trim_matrix(const DevCsc& A, DevCsc& out, Scratch& sc, cudaStream_t 
         out.cap = A.nnz;
     }
     trim_count_kernel<<<grid_for(nout, 256), 256, 0, s>>>(nout, A.colptr, A.rowind, cnt);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(exclusive_scan_i32_to_i32(cnt, out.colptr, nout, tmp, s));
     int32_t nnz = 0;
     RCHOL_TRY(cudaMemcpyAsync(&nnz, out.colptr + nout, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     trim_scatter_kernel<<<grid_for(nout, 256), 256, 0, s>>>(nout, A.colptr, A.rowind, A.val, out.colptr,
                                                             out.rowind, out.val);
+    count_launch();
     RCHOL_TRY(cudaGetLastError());
     RCHOL_TRY(cudaStreamSynchronize(s));
     out.nnz = nnz;

@@ -173,9 +173,11 @@ cudaError_t stable_key_order_carried(const int32_t* key, int32_t n, int32_t nkey
         int32_t* out = ((passes - 1 - p) % 2 == 0) ? order : buf;
         int32_t* kout = p + 1 < passes ? (p % 2 == 0 ? kb0 : kb1) : nullptr;
         radix_hist_carried_kernel<<<ntiles, kSortThreads, 0, s>>>(kin, n, 8 * p, ntiles, hist);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
         RCHOL_TRY(exclusive_scan_i32_to_i32(hist, offs, nh, tmp, s));
         radix_scatter_carried_kernel<<<ntiles, kSortThreads, 0, s>>>(kin, in, n, 8 * p, ntiles, offs, kout, out);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
         in = out;
         kin = kout;
@@ -213,9 +215,11 @@ cudaError_t stable_key_order_from(const int32_t* key, const int32_t* in0, int32_
     for (int p = 0; p < passes; ++p) {
         int32_t* out = ((passes - 1 - p) % 2 == 0) ? order : buf;
         radix_hist_kernel<<<ntiles, kSortThreads, 0, s>>>(key, in, n, 8 * p, ntiles, hist);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
         RCHOL_TRY(exclusive_scan_i32_to_i32(hist, offs, nh, tmp, s));
         radix_scatter_kernel<<<ntiles, kSortThreads, 0, s>>>(key, in, n, 8 * p, ntiles, offs, out);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
         in = out;
     }

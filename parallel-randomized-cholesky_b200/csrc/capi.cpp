@@ -698,6 +698,7 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     *out = nullptr;
     if (!ctx->have) return fail(ctx, RCHOL_ERR_NO_MATRIX, "no matrix loaded");
     cudaSetDevice(ctx->device);
+    const int64_t launches0 = rchol::t_launches;
     const rchol_opts& o = ctx->o;
     const int block = 32 * o.warps_per_block;
     const int max_grid = rchol::factor_resident_grid(block, o.slab_entries, ctx->device);
@@ -823,10 +824,7 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     info.solve_depth_b = f->F.depth_b;
     info.bwd_head_levels = f->F.hb_nlev;
     info.bwd_head_rows = f->F.hb_rows;
-    // setup (count, 3-pass scan, scatter, queue) + elimination + assembly
-    // (counts, scans, scatter, transpose, maxima, row sorts, level order)
-    info.kernel_launches = 6 + 1 + 1 + 3 + 1 + 3 + 1 + 2 + 1 + 1 + 1 + 3 + 1 +
-                           (o.precision == RCHOL_PREC_FP32_FACTOR ? 3 : 0);
+    info.kernel_launches = (int)(rchol::t_launches - launches0);
     info.lc_ptr = reinterpret_cast<const long long*>(f->F.lc_ptr);
     info.lc_idx = f->F.lc_idx;
     info.lc_val = f->F.lc_val;
@@ -836,10 +834,6 @@ extern "C" rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out) {
     info.diag = f->F.diag;
     info.fills = (long long)c64[1];
     info.tail_vertices = std::min<int32_t>(std::max(0, o.tail_vertices), ctx->A.n);
-    if (info.tail_vertices > 0) ++info.kernel_launches;
-    // narrow levels: both level tables, then (when built) their slab indices
-    if (o.exact_bwd_levels && o.bwd_head)
-        info.kernel_launches += 2 + (f->F.nf_rows > 0 ? 1 : 0) + (f->F.nb_rows > 0 ? 2 : 0);
     f->info = info;
     *out = f;
     return RCHOL_OK;

@@ -2031,8 +2031,10 @@ static cudaError_t count_lower(const DevCsc& A, int32_t* lower_cnt, int32_t* dep
     cudaError_t e = cudaMemsetAsync(huge, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
     count_lower_kernel<<<grid_for(A.n, 256), 256, 0, s>>>(A.n, A.colptr, A.rowind, lower_cnt, dep, huge);
+    count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     count_huge_kernel<<<2 * current_sm_count(), 256, 0, s>>>(A.colptr, A.rowind, huge, lower_cnt, dep);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -2048,6 +2050,7 @@ cudaError_t launch_lower_and_deps(const DevCsc& A, FactorWork& w, cudaStream_t s
     if (e != cudaSuccess) return e;
     scatter_lower_kernel<<<grid_for(A.n, 256), 256, 0, s>>>(A.n, A.colptr, A.rowind, A.val, w.lcolptr, w.lrow,
                                                              w.lval);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -2063,8 +2066,10 @@ cudaError_t launch_init_factor_state(FactorWork& w, cudaStream_t s) {
     if ((e = cudaMemsetAsync(w.hlock, 0, sizeof(int32_t) * w.nhuge, s)) != cudaSuccess) return e;
     prefill_bucket_kernel<<<grid_for(w.n, 256), 256, 0, s>>>(w.n, w.c0, w.lcolptr, w.lrow, w.lval,
                                                                             w.fcnt, w.brow, w.bval);
+    count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     init_queue_kernel<<<grid_for(w.n, 256), 256, 0, s>>>(w.n, w.dep, w.queue, w.counters);
+    count_launch();
     return cudaGetLastError();
 }
 
@@ -2142,6 +2147,7 @@ cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s
     if (e != cudaSuccess) return e;
     if (mid > 0) {
         factor_kernel<<<cfg.grid, cfg.block, smem, s>>>(a);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     if (mid < tail) {
@@ -2149,6 +2155,7 @@ cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s
         RCHOL_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CtaMid::kBytes));
         factor_cta_kernel<256, 4><<<std::min<int32_t>(cfg.cta_grid, tail - mid), 256, CtaMid::kBytes, s>>>(
             a, mid, tail, kMidTicket);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     if (tail < w.n) {
@@ -2156,6 +2163,7 @@ cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s
         RCHOL_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, CtaTail::kBytes));
         factor_cta_kernel<1024, 4><<<std::min<int32_t>(current_sm_count(), w.n - tail), 1024, CtaTail::kBytes, s>>>(
             a, tail, w.n, kTailTicket);
+        count_launch();
         RCHOL_TRY(cudaGetLastError());
     }
     return cudaSuccess;

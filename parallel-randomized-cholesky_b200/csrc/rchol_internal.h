@@ -62,6 +62,11 @@ struct Scratch {
     }
 };
 
+// Kernels launched by the calling thread on the factorization's path (set-up,
+// elimination, scans, sorts, assembly, schedules), counted where they are launched.
+extern thread_local int64_t t_launches;
+inline void count_launch() { ++t_launches; }
+
 // Error codes written to the device status word (first writer wins).
 enum DeviceError : int {
     kDevOk = 0,

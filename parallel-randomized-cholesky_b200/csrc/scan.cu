@@ -5,6 +5,8 @@
 
 namespace rchol {
 
+thread_local int64_t t_launches = 0;
+
 namespace {
 
 constexpr int kScanBlock = 256;
@@ -91,8 +93,11 @@ cudaError_t exclusive_scan(const int32_t* in, OutT* out, int64_t n, void* tmp, c
     int64_t ntiles = ceil_div(n > 0 ? n : 1, kTile);
     long long* ts = reinterpret_cast<long long*>(tmp);
     tile_sum_kernel<<<(unsigned)ntiles, kScanBlock, 0, s>>>(in, n, ts);
+    count_launch();
     scan_tile_sums_kernel<<<1, kScanBlock, 0, s>>>(ts, ntiles);
+    count_launch();
     tile_scan_kernel<OutT><<<(unsigned)ntiles, kScanBlock, 0, s>>>(in, n, ts, out);
+    count_launch();
     return cudaGetLastError();
 }
 

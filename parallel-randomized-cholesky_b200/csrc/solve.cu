@@ -2154,9 +2154,11 @@ cudaError_t pcg_solve(PcgSolver* s, const double* dB, double* dX, SolveResult* r
     SolveArgs a = s->args(dB, dX);
     if ((e = s->launch(s->k_init, s->grid_vec, a)) != cudaSuccess) return e;
     if ((e = s->launch_start(dB, dX)) != cudaSuccess) return e;
-    // per iteration: SpMV, forward, backward (+ the backward head)
-    const int per_it = 3 + (s->use_narrow() ? 1 : 0) + (s->n_lrows > 0 ? 1 : 0);
-    res->kernel_launches += per_it;
+    // a start: set-up, forward, backward (+ the narrow levels); an iteration: the
+    // SpMV (+ its long rows) in place of the set-up
+    const int per_start = 3 + (s->use_narrow() ? 1 : 0);
+    const int per_it = per_start + (s->n_lrows > 0 ? 1 : 0);
+    res->kernel_launches += per_start;
     if ((e = cudaEventRecord(s->ev1, s->stream)) != cudaSuccess) return e;
     int restarts = 0;
     while (true) {
@@ -2216,7 +2218,7 @@ cudaError_t pcg_solve(PcgSolver* s, const double* dB, double* dX, SolveResult* r
             cudaSuccess)
             return e;
         if ((e = s->launch_start(dB, dX)) != cudaSuccess) return e;
-        res->kernel_launches += per_it + 1;
+        res->kernel_launches += per_start + 1;  // the true residual and the restart, no set-up
     }
     if ((e = cudaEventRecord(s->ev2, s->stream)) != cudaSuccess) return e;
     if ((e = cudaEventSynchronize(s->ev2)) != cudaSuccess) return e;

@@ -358,6 +358,24 @@ def test_overflow_chunks_claimed_once(n, edges, tail):
     assert info.chunks_used == units and units > 0
 
 
+def test_kernel_launches_follow_the_passes():
+    """info.kernel_launches counts the passes that a factorization runs: a warp
+    a vertex, then 256 threads a vertex for the last eighth (none of fewer than 8
+    vertices), then 1024 threads for a tail; the planning of narrow levels
+    launches nothing when there are too few levels."""
+    def launches(n, r, c, v, g, **opts):
+        return _gpu_factor(n, r, c, v, g, 5, **opts)[1].kernel_launches
+
+    m = grid_laplacian((20, 20), seed=5)
+    n = m[0]
+    two = launches(*m, bwd_head=0)
+    assert launches(*m, bwd_head=0, tail_vertices=4) == two + 1
+    assert launches(*m, bwd_head=0, tail_vertices=n // 2) == two
+    tiny, less = grid_laplacian((7,), seed=5), grid_laplacian((8,), seed=5)
+    assert launches(*less, bwd_head=0) == launches(*tiny, bwd_head=0) + 1
+    assert launches(*tiny, bwd_head=1) == launches(*tiny, bwd_head=0)
+
+
 @pytest.mark.parametrize("length", [64, 255, 256, 257, 511, 513, 1100])
 def test_lower_triangle_of_long_columns(length):
     """A hub in the middle of the order, its column `length` entries long and
