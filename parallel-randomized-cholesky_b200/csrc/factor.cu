@@ -2137,8 +2137,8 @@ cudaError_t launch_factor(FactorWork& w, const FactorLaunch& cfg, cudaStream_t s
     a.smem_region = smem_region_bytes(cfg.smem_slab);
     a.timeout_ns = (unsigned long long)(cfg.timeout_s * 1e9);
     // [0, mid) a warp per vertex, [mid, tail) a 256-thread CTA, [tail, n) a
-    // 1024-thread CTA (a tail of every vertex keeps the warp path for none)
-    const int32_t tail = cfg.tail > 0 && cfg.tail < w.n ? w.n - cfg.tail : w.n;
+    // 1024-thread CTA (a tail of every vertex leaves none to the others)
+    const int32_t tail = w.n - std::min<int32_t>(w.n, std::max(0, cfg.tail));
     const int32_t mid = std::min<int32_t>(tail, w.n - std::min<int32_t>(w.n, cfg.cta));
     a.tail = mid;
     a.gsize = cfg.gsize;

@@ -376,6 +376,21 @@ def test_kernel_launches_follow_the_passes():
     assert launches(*tiny, bwd_head=1) == launches(*tiny, bwd_head=0)
 
 
+def test_tail_of_every_vertex_is_one_pass():
+    """tail_vertices >= n: every vertex is eliminated by a CTA of 1024 threads,
+    in one launch, bit-exact."""
+    n, r, c, v, g = grid_laplacian((30, 31), seed=8, excess_frac=0.05)
+    orc = OracleProblem(n, r, c, v, trim=g).factor(seed=5)
+    infos = []
+    for tail in (0, n, 2 * n):
+        gpu, info = _gpu_factor(n, r, c, v, g, 5, tail_vertices=tail)
+        _compare(gpu, orc)
+        infos.append(info)
+    assert [i.tail_vertices for i in infos] == [0, n, n]
+    # instead of a warp a vertex and 256 threads a vertex
+    assert [i.kernel_launches - infos[0].kernel_launches for i in infos] == [0, -1, -1]
+
+
 @pytest.mark.parametrize("length", [64, 255, 256, 257, 511, 513, 1100])
 def test_lower_triangle_of_long_columns(length):
     """A hub in the middle of the order, its column `length` entries long and
