@@ -216,6 +216,18 @@ rchol_status rchol_matrix_copy_to_host(const rchol_ctx* ctx, int* colptr, int* r
 /* ---- factorization (driver.cu:43-1302 kernel + :1309-1548 assembly) ---- */
 rchol_status rchol_factor(rchol_ctx* ctx, rchol_factor_t** out);
 rchol_status rchol_factor_get_info(const rchol_factor_t* f, rchol_factor_info* info);
+/* The rows that one cluster of CTAs solves for one right-hand side (bwd_head):
+ * the last rows of the forward schedule and the first of the backward one, all
+ * 0 where the levels were too few or too wide.  Reads the tasks back: for
+ * tests and tuning, not for a solve loop. */
+typedef struct rchol_narrow_info {
+    int max_rows;             /* the cluster's limit, for either direction */
+    int fwd_rows, fwd_tasks;  /* rows, warp tasks */
+    int fwd_parts;            /* tasks that are parts of split rows */
+    int bwd_rows, bwd_tasks, bwd_parts;
+    int long_form;            /* 1: the kernel's form for rows of many slots a lane */
+} rchol_narrow_info;
+rchol_status rchol_factor_narrow(const rchol_factor_t* f, rchol_narrow_info* info);
 /* Strict CSC of L (colptr[n+1], rowind/val[nnz_strict]) and D[n] to the host. */
 rchol_status rchol_factor_copy_to_host(const rchol_factor_t* f, long long* colptr, int* rowind, double* val,
                                        double* diag);

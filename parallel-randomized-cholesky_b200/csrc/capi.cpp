@@ -845,6 +845,31 @@ extern "C" rchol_status rchol_factor_get_info(const rchol_factor_t* f, rchol_fac
     return RCHOL_OK;
 }
 
+extern "C" rchol_status rchol_factor_narrow(const rchol_factor_t* f, rchol_narrow_info* info) {
+    if (!f || !info) return RCHOL_ERR_INVALID;
+    rchol_ctx* ctx = f->ctx;
+    const DevFactor& F = f->F;
+    std::memset(info, 0, sizeof(*info));
+    info->max_rows = rchol::kNarrowRows;
+    info->fwd_rows = F.nf_rows;
+    info->fwd_tasks = F.nf_rows > 0 ? F.npt_f - F.nf_task : 0;
+    info->bwd_rows = F.nb_rows;
+    info->bwd_tasks = F.nb_task;
+    info->long_form = F.narrow_long ? 1 : 0;
+    cudaSetDevice(f->device);
+    std::vector<int4> d((size_t)std::max(info->fwd_tasks, info->bwd_tasks));
+    for (int dir = 0; dir < 2; ++dir) {
+        const int nt = dir ? info->bwd_tasks : info->fwd_tasks;
+        if (nt == 0) continue;
+        CK(cudaMemcpy(d.data(), dir ? F.pack_b : F.pack_f + F.nf_task, sizeof(int4) * (size_t)nt,
+                      cudaMemcpyDeviceToHost), "copy tasks");
+        int parts = 0;
+        for (int t = 0; t < nt; ++t) parts += (d[(size_t)t].z >> 11) & 1;
+        (dir ? info->bwd_parts : info->fwd_parts) = parts;
+    }
+    return RCHOL_OK;
+}
+
 extern "C" rchol_status rchol_factor_copy_to_host(const rchol_factor_t* f, long long* colptr, int* rowind,
                                                   double* val, double* diag) {
     if (!f) return RCHOL_ERR_INVALID;

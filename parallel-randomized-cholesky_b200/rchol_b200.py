@@ -36,7 +36,7 @@ EXPORTS = sorted([
     "rchol_prepare_and_solve", "rchol_generate", "rchol_free_host", "rchol_write_mtx", "rchol_batch_set",
     "rchol_batch_solve", "rchol_zero_sum_vector", "rchol_set_sddm", "rchol_write_bin", "rchol_read_bin",
     "rchol_save_bin", "rchol_load_bin", "rchol_autotune", "rchol_ordering",
-    "rchol_hop_latency",
+    "rchol_hop_latency", "rchol_factor_narrow",
 ])
 
 
@@ -67,6 +67,11 @@ class FactorInfo(C.Structure):
                 ("lr_ptr", C.c_void_p), ("lr_idx", C.c_void_p), ("lr_val", C.c_void_p), ("diag", C.c_void_p),
                 ("tail_vertices", C.c_int), ("solve_depth_b", C.c_int), ("bwd_head_levels", C.c_int),
                 ("bwd_head_rows", C.c_int)]
+
+
+class NarrowInfo(C.Structure):
+    _fields_ = [("max_rows", C.c_int), ("fwd_rows", C.c_int), ("fwd_tasks", C.c_int), ("fwd_parts", C.c_int),
+                ("bwd_rows", C.c_int), ("bwd_tasks", C.c_int), ("bwd_parts", C.c_int), ("long_form", C.c_int)]
 
 
 class TuneResult(C.Structure):
@@ -123,6 +128,7 @@ def lib():
         L.rchol_matrix_copy_to_host.argtypes = [vp, vp, vp, vp]
         L.rchol_factor.argtypes = [vp, C.POINTER(vp)]
         L.rchol_factor_get_info.argtypes = [vp, C.POINTER(FactorInfo)]
+        L.rchol_factor_narrow.argtypes = [vp, C.POINTER(NarrowInfo)]
         L.rchol_factor_copy_to_host.argtypes = [vp, vp, vp, vp, vp]
         L.rchol_factor_write.argtypes = [vp, C.c_char_p]
         L.rchol_factor_read.argtypes = [vp, C.c_char_p, C.POINTER(vp)]
@@ -306,6 +312,12 @@ class Factor:
         fi = FactorInfo()
         _check(lib().rchol_factor_get_info(self.h, C.byref(fi)))
         return fi
+
+    def narrow(self):
+        """The rows that one cluster solves for one right-hand side."""
+        ni = NarrowInfo()
+        _check(lib().rchol_factor_narrow(self.h, C.byref(ni)))
+        return ni
 
     def to_host(self):
         """Strict CSC of L (rows ascending, values L_ij) and D."""

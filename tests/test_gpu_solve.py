@@ -552,3 +552,98 @@ def test_backward_levels_of_long_columns(m):
         lev[j] = 1 + lev[below].max() if below.size else 0
     assert int(np.diff(cp).max()) >= m - 1
     assert depth == lev.max() + 1
+
+
+def _complete_graph(m):
+    r, c = np.triu_indices(m, 1)
+    w = np.random.default_rng(m).uniform(1.0, 2.0, r.size)
+    d = np.bincount(r, w, m) + np.bincount(c, w, m)
+    i = np.arange(m)
+    return m, np.concatenate([r, c, i]), np.concatenate([c, r, i]), np.concatenate([-w, -w, d]), False
+
+
+def _paths(count, length):
+    """`count` paths side by side, vertex l * count + p the l-th of path p, each
+    vertex with a small diagonal excess."""
+    n = count * length
+    a, i = np.arange(n - count), np.arange(n)
+    w = np.random.default_rng(1).uniform(1.0, 2.0, a.size)
+    d = np.bincount(a, w, n) + np.bincount(a + count, w, n) + 1e-3
+    g, e = np.full(n, n), np.full(n, -1e-3)
+    return (n + 1, np.concatenate([a, a + count, i, i, g, [n]]), np.concatenate([a + count, a, i, g, i, [n]]),
+            np.concatenate([-w, -w, d, e, e, [n * 1e-3]]), True)
+
+
+NARROW = {
+    # rows a level times levels outgrow the cluster's memory
+    "paths": (lambda: _paths(1000, 40), dict(fwd_rows=26000, bwd_rows=26000, long_form=0)),
+    # every row inside; rows and columns long and split
+    "complete600": (lambda: _complete_graph(600), dict(fwd_rows=600, bwd_rows=600, long_form=1, fwd_parts=0)),
+    "complete1300": (lambda: _complete_graph(1300), dict(fwd_rows=1300, bwd_rows=1300, long_form=1)),
+    # split forward rows, long form
+    "power_law": (lambda: R.generate("chunglu", [100000, 1000000, 2, 20000], wlo=1.0, whi=10.0, seed=7),
+                  dict(long_form=1)),
+    # wide levels outside, short form
+    "cube": (lambda: grid_laplacian((40, 41, 42), seed=5, excess_frac=0.05), dict(long_form=0)),
+}
+SPLIT = {"complete600": (0, 1), "complete1300": (1, 1), "power_law": (1, 0)}  # forward, backward
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+@pytest.mark.parametrize("graph", sorted(NARROW))
+def test_narrow_ranges_are_taken_and_match(graph, fp32):
+    """The cluster kernel does take the rows that these graphs are meant to give
+    it (each kind of range, both forms, split rows), z equals the persistent
+    kernels' bit for bit, and two PCG iterations agree to rounding: the forms
+    differ only in how r.z is grouped."""
+    make, want = NARROW[graph]
+    n, r, c, v, g = make()
+    zs, xs = [], []
+    for narrow in (0, 1):
+        ctx = R.Context(seed=6, precision=R.PREC_FP32_FACTOR if fp32 else R.PREC_FP64, bwd_head=narrow, tol=1e-12,
+                        max_iter=2)
+        try:
+            ctx.set_triplets(n, r, c, v, trim_ground=g)
+            f = ctx.factor()
+            ni = f.narrow()
+            if not narrow:
+                assert ni.fwd_rows == ni.bwd_rows == ni.fwd_tasks == ni.bwd_tasks == 0
+            else:
+                assert 0 < ni.fwd_rows <= ni.max_rows and 0 < ni.bwd_rows <= ni.max_rows
+                assert {k: getattr(ni, k) for k in want} == want
+                assert (int(ni.fwd_parts > 0), int(ni.bwd_parts > 0)) == SPLIT.get(graph, (0, 0))
+            b = zero_sum_normal(f.info().n, 8)
+            zs.append(ctx.precond_apply(f, b, fp32=fp32))
+            xs.append(ctx.pcg_solve(f, b))
+            f.free()
+        finally:
+            ctx.close()
+    np.testing.assert_array_equal(zs[1], zs[0])
+    (x0, i0), (x1, i1) = xs
+    np.testing.assert_allclose(x1, x0, rtol=0, atol=1e-12 * np.abs(x0).max())
+    assert i1["kernel_launches"] > i0["kernel_launches"]
+
+
+def test_narrow_waits_end_and_recover():
+    """A graph whose rows the cluster kernel solves all, with a wait limit far
+    below its time: its own waits run out, the call reports a timeout, and
+    the next one with a normal limit gives the bits it gave before."""
+    n, r, c, v, g = _complete_graph(600)
+    ctx = R.Context(seed=6, precision=R.PREC_FP64)
+    try:
+        ctx.set_triplets(n, r, c, v, trim_ground=g)
+        f = ctx.factor()
+        assert f.narrow().fwd_rows == f.narrow().bwd_rows == n
+        b = zero_sum_normal(n, 8)
+        z = ctx.precond_apply(f, b)
+        ctx.set_opts(timeout_s=1e-7)
+        for call in (ctx.precond_apply, ctx.pcg_solve):
+            with pytest.raises(R.RcholError) as e:
+                call(f, b)
+            assert e.value.status == 5
+        ctx.set_opts(timeout_s=30.0)
+        np.testing.assert_array_equal(ctx.precond_apply(f, b), z)
+        assert ctx.pcg_solve(f, b)[1]["converged"]
+        f.free()
+    finally:
+        ctx.close()
