@@ -187,22 +187,22 @@ __device__ void block_partials_lane(double v, double* out_block /* [K] */) {
     __syncthreads();
 }
 
-// Returns true in exactly one thread of the last block to finish; that block
-// then reduces the partials.  `ticket` is reset for the next use.
+// Returns true in the threads of the last block to finish; that block then
+// reduces the partials.  `ticket` is reset for the next use.  The fences stand
+// with the ticket, in one thread between two barriers: so they order what all
+// threads of a block wrote before its ticket, and the last ticket before what all
+// threads of the last block read.
 __device__ __forceinline__ bool last_block(unsigned* ticket) {
     __shared__ bool is_last;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+        __threadfence();
         unsigned t = atomicAdd(ticket, 1u);
         is_last = (t == gridDim.x - 1);
+        __threadfence();
     }
     __syncthreads();
-    if (is_last) {
-        __threadfence();
-        return true;
-    }
-    return false;
+    return is_last;
 }
 
 // Column sums of the blocks' partials in block order.  The last block brings

@@ -25,3 +25,16 @@ def test_counters_drop_after_barrier_then_fence():
         barrier = max(before.rfind("__syncthreads"), before.rfind("__syncwarp"))
         fence = before.rfind("__threadfence()")
         assert 0 <= barrier < fence, text[barrier:at]
+
+
+def test_block_tickets_are_taken_between_fences():
+    """The last block of a reduction reads what every thread of the other blocks
+    wrote: barrier, fence, ticket, fence, barrier, the fences in the thread that
+    takes the ticket."""
+    text = code("solve.cu")
+    at = text.index("bool last_block(")
+    body = text[at:text.index("\n}", at)]
+    steps = re.findall(r"__syncthreads|__threadfence|atomicAdd", body)
+    assert steps == ["__syncthreads", "__threadfence", "atomicAdd", "__threadfence", "__syncthreads"]
+    lead = body[body.index("if (threadIdx.x == 0) {"):body.rindex("__syncthreads")]
+    assert lead.count("__threadfence") == 2 and "atomicAdd" in lead
