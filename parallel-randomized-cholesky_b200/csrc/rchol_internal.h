@@ -300,7 +300,8 @@ cudaError_t build_solve_layouts(DevFactor& f, Scratch& sc, cudaStream_t s);
 // up to kNarrowRows rows a direction (each CTA's shared memory holds a copy of
 // their values: 208 of the 227 KB), in levels of at most kNarrowTasks tasks;
 // fewer than kNarrowMinLevels such levels stay with the persistent kernels.
-// 128 tasks: half the cluster's warps.  Against 256 the 256^2 solve takes 6.26
+// 128 tasks: half the warps of the short form, all of the long form's (8 fewer
+// where CTA 0 adds r.z).  Against 256 the 256^2 solve takes 6.26
 // and 6.32 ms, 61x53x47 the same, one 128^3 apply 1.01 and 1.10; 64 was slower than
 // 256 in an earlier form of the kernel (256^2 7.0 against 6.8, 61x53x47 13.2 against
 // 12.4).  16 CTAs against 4 (64 tasks) and 1 (16 tasks): 256^2 6.3 / 7.0 / 7.7 ms;
@@ -315,8 +316,10 @@ bool narrow_fits();  // the current device holds such a cluster
 // The rows whose r.z terms are summed apart (DevFactor::hb_nlev): the
 // backward levels from the first while each holds at most kHeadMaxRows rows,
 // kHeadParts tasks and no part task, and head_bytes of them stays within
-// kHeadBytes.  The sum's grouping, and so the last bits of every iterate,
-// follows these limits.
+// kHeadBytes.  The limits are those of a kernel that is gone, one CTA that solved
+// these levels with their tasks, slabs and rows staged in its shared memory;
+// no kernel's needs today.  They stay because the sum's grouping, and so the last
+// bits of every iterate, follows them.
 constexpr int kHeadParts = 16;
 constexpr int kHeadMinLevels = 8;
 constexpr int kHeadMaxRows = 1024;
@@ -376,9 +379,9 @@ cudaError_t trim_matrix(const DevCsc& A, DevCsc& out, Scratch& sc, cudaStream_t 
         if (e__ != cudaSuccess) return e__; \
     } while (0)
 
-// Shared large slabs of the elimination kernel: between kHugeSlabsMin and
-// kHugeSlabsMax (as many as fit kHugeSlabBudget bytes); the cooperative
-// tail runs one CTA per slab.
+// Shared large slabs of the elimination kernels, taken under a lock by the warp
+// or CTA whose list needs one: between kHugeSlabsMin and kHugeSlabsMax (as many
+// as fit kHugeSlabBudget bytes).
 constexpr int kHugeSlabsMin = 8;
 constexpr int kHugeSlabsMax = 32;
 constexpr size_t kHugeSlabBudget = size_t(512) << 20;

@@ -48,7 +48,7 @@ struct PcgScalars {
     int phase;               // 0: the next bwd pass initialises rz (start/restart)
     int status;              // device error code
     unsigned ticket[4];
-    double hrz;              // r.z over the backward head's rows
+    double hrz;              // r.z over the first hb_nlev backward levels
 };
 
 namespace {
@@ -211,9 +211,11 @@ __device__ __forceinline__ bool last_block(unsigned* ticket) {
 // 1184 partials of a SpMV launch took 10 of its 23 us on 2867 unknowns.  (A tree
 // would be faster still, but any other grouping moves the iterates of loosely
 // converged solves by up to their error.)  The tile is small because a kernel's
-// shared memory comes out of the L1 that its gathers live in: with 8 KB instead
-// of 4 the k = 8 SpMV took 72 us, not 60; 32 columns need the larger tile (258
-// against 283 us).
+// shared memory comes out of the L1 that its gathers live in; from 16 columns on
+// 8 KB against 4 give the SpMV 145 / 257 us (k = 16 / 32) against 155 / 281 on a 27-point
+// 64^3 matrix and 114 / 201 against 107 / 194 on a 7-point 75x71x69, although the
+// two tiles in registers spill 36-40 bytes of the 32 registers there; for 2 to 8
+// columns both are the same.
 template <int K>
 constexpr int sum_tile() {
     return K >= 16 ? 1024 : 512;
@@ -879,7 +881,8 @@ constexpr int kPackM = 4;  // slab slots per lane held in registers
 #define RCHOL_TRICKLE 2
 #endif
 constexpr unsigned kTrickle = RCHOL_TRICKLE;
-// 3 CTAs of 256 threads per SM (80 registers, no spills in the poll loops)
+// 3 CTAs of 256 threads per SM (80 registers; with FP64 values the forward kernel
+// spills 28 and the backward one 52 bytes, with FP32 values 0 and 12)
 #ifndef RCHOL_PACK_MINB
 #define RCHOL_PACK_MINB 3
 #endif
